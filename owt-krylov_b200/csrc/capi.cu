@@ -361,9 +361,13 @@ void store_factors(Preconditioner& p)
     if (p.storage == OWTK_F32) {
         kern::convert<float, double>(c, nv, p.d_fvalues.as<double>(), p.lp_vals.as<float>());
         kern::convert<float, double>(c, ni, p.inv_diag.as<double>(), p.lp_inv.as<float>());
+        if (p.upper_local.ready) kern::local_ilu_pack<float, float>(c, p, p.lp_vals.as<float>(), p.lp_inv.as<float>());
     } else {
         kern::convert<__nv_bfloat16, double>(c, nv, p.d_fvalues.as<double>(), p.lp_vals.as<__nv_bfloat16>());
         kern::convert<__nv_bfloat16, double>(c, ni, p.inv_diag.as<double>(), p.lp_inv.as<__nv_bfloat16>());
+        if (p.upper_local.ready)
+            kern::local_ilu_pack<float, __nv_bfloat16>(c, p, p.lp_vals.as<__nv_bfloat16>(),
+                                                       p.lp_inv.as<__nv_bfloat16>());
     }
 }
 
@@ -1031,15 +1035,26 @@ std::unique_ptr<owtk_preconditioner> make_pc(owtk_matrix* m, owtk_pc_kind kind, 
         levels_of(m->owned, m->h_rowptr.data(), cols.data(), lower, upper);
         build_sweep(*p->ctx, p->lower, m->owned, m->bs, lower, false);
         build_sweep(*p->ctx, p->upper, m->owned, m->bs, upper, true);
+        if (const int warps = local_sweep_warps(*p->ctx, p->lower, p->upper, m->owned, m->bs)) {
+            const std::int32_t* rp = m->h_rowptr.data();
+            build_local_sweep(*p->ctx, *p, warps, es, rp, rp + 1, rp, rp + 1, cols.data(), true);
+        }
         break;
     }
     case OWTK_PC_ILU: {
         if (m->kind != 0) fail(OWTK_ERR_INVALID_ARGUMENT, "ILU needs a component-diagonal BSR matrix");
         if (!(parameter >= 0)) fail(OWTK_ERR_INVALID_ARGUMENT, "ILU fill level must be >= 0");
         ilu_symbolic(*p, *m, static_cast<std::size_t>(parameter));
-        if (storage == OWTK_F64 && m->bs <= 32 && !p->chain.ready) {
-            const char* env = std::getenv("OWTK_PACKED_SWEEP");   // 0: applies read the factor in place
-            if (!env || std::atoi(env) != 0) {
+        const char* env = std::getenv("OWTK_PACKED_SWEEP");   // 0: applies read the factor in place
+        const bool in_place = env && std::atoi(env) == 0;
+        const bool scheduled = in_place || p->chain.ready || p->l_lower.ready || p->c_lower.ready;
+        if (const int warps = scheduled ? 0 : local_sweep_warps(*p->ctx, p->lower, p->upper, m->owned, m->bs)) {
+            const std::size_t ls = storage == OWTK_F64 ? es : sizeof(float);
+            const std::int32_t *rp = p->f_rowptr.data(), *dp = p->f_diagpos.data(), *ci = p->f_cols.data();
+            build_local_sweep(*p->ctx, *p, warps, ls, rp, dp, dp, rp + 1, ci, false);
+        }
+        if (storage == OWTK_F64 && m->bs <= 32 && !p->chain.ready && !p->upper_local.ready) {
+            if (!in_place) {
                 pack_sweep(*p->ctx, p->lower, m->bs, es, p->f_rowptr, p->f_cols, p->f_diagpos, false);
                 pack_sweep(*p->ctx, p->upper, m->bs, es, p->f_rowptr, p->f_cols, p->f_diagpos, true);
             }

@@ -1,0 +1,702 @@
+// Triangular sweeps with one CTA per component (sm_100a): the ILU and SSOR
+// applies of component-diagonal matrices.
+//
+// What bounds a sweep is the hand-off from a level to the next one: about
+// 0.85 us when the value travels through L2 from one SM to another
+// (kernels_sweep.cu).  The components of a component-diagonal matrix never
+// meet, so each can be solved by a CTA of its own, and inside a CTA a level
+// ends with a barrier and its values travel through shared memory.  The price
+// is that one SM does all the rows of a component, so this path is taken while
+// the levels are narrow enough for that (local_sweep_warps).
+//
+// A level's rows are cut into steps of up to W tasks, a task being up to 32
+// rows, one per lane; a team of W warps takes a step, and T teams take the
+// steps in turn.  Step s waits for step s - 1 at a named barrier that team s - 1
+// arrives at and team s waits at, so all a step leaves between two barriers is
+// its shared-memory reads, its sums and one store.  A task's operands come by
+// asynchronous copies, kDepth of the warp's tasks ahead, issued while the other
+// teams have the barrier: loads into registers do not stay in flight that long
+// (the same kernel with them took 0.95 us a level at 250 rows, however deep the
+// pipeline).  Nothing polls: warps polling shared memory for a sentinel took
+// 310 ns a level at 17 rows and 0.95 us at 250, the polls taking the issue
+// slots.  One ILU(0) apply, FP64, before (all SMs, levels through L2) and now:
+//   4,096 rows, 17 a level: 350 -> 47 us (W 1); 50,000 rows, 58 a level:
+//   1,390 -> 235 us (W 2); 200,000 rows, 115 a level: 2,880 -> 700 us (W 4);
+//   1,000,000 rows, 252 a level: 6,780 -> 3,270 us (W 4).
+// A step of one warp costs 75 ns, of two 95, of four 145: the wide steps are
+// bound by shared-memory wavefronts (about 80 a task: the gathers of the
+// results, and the operands once in and once out), which is also why eight
+// warps a team are slower than four.
+//
+// Results live in a shared-memory ring in step order, and a dependency is a
+// 16-bit ring slot.  One further back than the ring reaches is final in global
+// memory long before; it is copied into the task's stage like its operands (a
+// row of a low level may be read thousands of levels later: at 490,000 rows,
+// RCM order, 0.2% of the rows have such a dependency in the forward sweep).  Tasks with rows
+// of more than kHold dependencies, or more than 32 far ones, read 32-bit codes
+// and the far values in place instead.  Absent dependencies read
+// a slot that holds zero with a zero coefficient, which leaves every y, -0 and
+// NaN included, as it is.
+//
+// Per (row, component) the arithmetic is the reference's
+// (preconditioner.hpp:165-247, :320-363), term by term in entry order with
+// explicit rounding, so results equal the CPU path bit for bit.
+
+#include <algorithm>
+#include <cstdlib>
+#include <type_traits>
+
+#include <cuda_bf16.h>
+
+#include "device_common.cuh"
+#include "owtk_internal.h"
+
+namespace owtk {
+namespace {
+
+using namespace dev;
+
+constexpr int kHold = 8;              // dependencies held in registers
+constexpr int kTaskEntries = 192;     // padded entries of a task that is staged
+constexpr int kDepth = 2;             // tasks a warp has in flight (3 and 4: the same times)
+constexpr int kSharedBytes = 226 * 1024;
+// Teams by warps per team: as many as shared memory leaves a ring for and, at
+// four warps, as registers allow (at 1,000,000 rows 4, 5 and 6 teams of four
+// took 4,150, 3,730 and 3,260 us).
+constexpr int kTeams1 = 12, kTeams2 = 12, kTeams4 = 6;
+// A task's packed word: rows, width << 8, and
+constexpr int kFarFlag = 1 << 24;     // some dependencies are staged from global memory
+constexpr int kSlowFlag = 1 << 25;    // the slower form
+constexpr int kFarSlot = 0xffe0;      // slots from here on: the task's far values
+constexpr int kMaxEntries = 1 << 30;
+
+template<class T> struct Bits;
+template<> struct Bits<double> {
+    static __device__ __forceinline__ double quiet_nan() { return __longlong_as_double(0x7ff8000000000000ll); }
+};
+template<> struct Bits<float> {
+    static __device__ __forceinline__ float quiet_nan() { return __uint_as_float(0x7fc00000u); }
+};
+
+__device__ __forceinline__ void ld_ring(std::uint32_t a, double& v)
+{
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ld_ring(std::uint32_t a, float& v)
+{
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void st_ring(std::uint32_t a, double v)
+{
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_ring(std::uint32_t a, float v)
+{
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+template<int THREADS> __device__ __forceinline__ void bar_wait(int id)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(THREADS) : "memory");
+}
+template<int THREADS> __device__ __forceinline__ void bar_signal(int id)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(THREADS) : "memory");
+}
+
+__device__ __forceinline__ void copy16(std::uint32_t to, const void* from)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+}
+template<class T> __device__ __forceinline__ void copy_value(std::uint32_t to, const T* from)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to), "l"(from), "n"(sizeof(T)) : "memory");
+}
+
+// One direction of a sweep; arrays as in LocalSweep.
+template<class T>
+struct Direction {
+    const int4* task;        // [step][warp of the team]: first entry, first place, packed word, first ring slot
+    const std::uint16_t* slots;   // per entry: ring slot, or kFarSlot + k for the task's k-th far value
+    const int* far;          // [step][warp][32]: where the far values are (null: there are none)
+    const int* code;         // per entry: ring slot, or -1 - index of a far dependency (null: no slow task)
+    const int* to;           // per place: where its result goes (row, or place in the backward order)
+    const T* coef;           // per component and entry
+    const T* fin;            // per component and place: factor or divisor of the result
+    const T* in;             // per component and place
+    T* out;                  // forward: per component and place of the backward order; backward: the result
+    std::size_t entries, places, out_places;
+    int steps, ring, bs;
+};
+
+// A task's operands in shared memory.
+template<class T>
+struct __align__(16) Stage {
+    T coef[kTaskEntries];                // [dependency][row]
+    std::uint16_t slots[kTaskEntries];   // [dependency pair][row][2]
+    int to[32];
+    T own[32], fin[32], far[32];
+    int4 task;
+};
+
+static_assert(sizeof(Stage<double>) % 16 == 0 && sizeof(Stage<float>) % 16 == 0, "stages are copied in 16-byte pieces");
+
+// Where a lane copies a task's operands from, before the task's own offsets.
+template<class T>
+struct Source {
+    const T* coef;
+    const T* row;            // own (first lanes) or fin
+    const char* index;       // slots (24 lanes) or to
+    const T* far;            // result of the direction, for far values
+    std::size_t far_step;
+};
+
+template<class T, bool BACK>
+__device__ __forceinline__ Source<T> source_of(const Direction<T>& d, int lane, int c)
+{
+    constexpr int kPer = 16 / static_cast<int>(sizeof(T)), kRowLanes = 32 / kPer;
+    Source<T> s;
+    s.coef = d.coef + static_cast<std::size_t>(c) * d.entries + lane * kPer;
+    const std::size_t q = static_cast<std::size_t>(c) * d.places;
+    s.row = lane < kRowLanes ? d.in + q + lane * kPer : d.fin + q + (lane - kRowLanes) * kPer;
+    s.index = lane < 24 ? reinterpret_cast<const char*>(d.slots) + lane * 16
+                        : reinterpret_cast<const char*>(d.to) + (lane - 24) * 16;
+    s.far = d.out + (BACK ? static_cast<std::size_t>(c) : static_cast<std::size_t>(c) * d.out_places);
+    s.far_step = BACK ? d.bs : 1;
+    return s;
+}
+
+// Up to six copies a lane: a task's entries are contiguous and padded to 8,
+// its rows to 4.
+template<class T, bool FIN>
+__device__ __forceinline__ void load_operands(const Source<T>& s, int lane, int4 task, int far, std::uint32_t stage)
+{
+    constexpr int kSize = static_cast<int>(sizeof(T)), kPer = 16 / kSize, kRowLanes = 32 / kPer;
+    constexpr std::uint32_t kSlots = kTaskEntries * kSize, kOwn = kSlots + kTaskEntries * 2 + 128;
+    const int rows = task.z & 0xff;
+    if (rows > 0) {
+        const int entries = task.z & kSlowFlag ? 0 : rows * (task.z >> 8 & 0xff);
+        const T* coef = s.coef + task.x;
+        const std::uint32_t at = stage + lane * 16;
+#pragma unroll
+        for (int i = 0; i < kTaskEntries; i += 32 * kPer)
+            if (i + lane * kPer < entries) copy16(at + i * kSize, coef + i);
+        if (lane >= 24 || lane * 8 < entries)
+            copy16(at + kSlots, s.index + (lane < 24 ? static_cast<std::size_t>(task.x) * 2
+                                                     : static_cast<std::size_t>(task.y) * 4));
+        if (lane < (FIN ? 2 * kRowLanes : kRowLanes)) copy16(at + kOwn, s.row + task.y);
+        if (task.z & kFarFlag && far >= 0)
+            copy_value(stage + kOwn + (64 + lane) * kSize, s.far + static_cast<std::size_t>(far) * s.far_step);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The slower form: eight dependencies at a time, loaded when their turn comes.
+template<class T, bool BACK>
+__device__ __noinline__ T consume_slow(T y, const Direction<T>* dp, int lane, int c, int4 task, std::uint32_t ring)
+{
+    const Direction<T>& d = *dp;
+    const T* far = d.out + (BACK ? c : static_cast<std::size_t>(c) * d.out_places);
+    const std::size_t far_step = BACK ? d.bs : 1;
+    const int rows = task.z & 0xff, width = task.z >> 8 & 0xff, at = task.x + min(lane, rows - 1);
+    for (int j0 = 0; j0 < width; j0 += kHold) {
+        T x[kHold], coef[kHold];
+#pragma unroll
+        for (int j = 0; j < kHold; ++j) {
+            coef[j] = x[j] = T(0);
+            if (j0 + j < width) {
+                const std::size_t e = static_cast<std::size_t>(at) + (j0 + j) * rows;
+                const int code = __ldg(d.code + e);
+                coef[j] = __ldg(d.coef + static_cast<std::size_t>(c) * d.entries + e);
+                if (code >= 0) ld_ring(ring + code * static_cast<int>(sizeof(T)), x[j]);
+                else x[j] = __ldcg(far + static_cast<std::size_t>(-1 - code) * far_step);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kHold; ++j) y = sub_rn(y, mul_rn(coef[j], x[j]));
+    }
+    return y;
+}
+
+// One task of `N` padded dependencies: the operands from the stage, the wait
+// for the step before, the sums and the store that the next step waits for.
+// Straight-line between the barriers, because every instruction there is paid
+// once per step (uniform branches on the width there made a step of one warp
+// 250 cycles).  Returns the result of the lane's row.
+template<class T, int N, int PAIR, bool BACK, bool SSOR>
+__device__ __forceinline__ T run_task(const Stage<T>& h, const int4& task, int lane, std::uint32_t ring,
+                                      std::uint32_t slot, bool wait, bool signal, int wait_id, int signal_id)
+{
+    constexpr int kSize = static_cast<int>(sizeof(T));
+    const int rows = task.z & 0xff, l = min(lane, rows - 1);
+    const bool live = lane < rows;
+    std::uint32_t at[N > 0 ? N : 1];
+    T coef[N > 0 ? N : 1], x[N > 0 ? N : 1];
+#pragma unroll
+    for (int j = 0; j < N; j += 2) {
+        const unsigned pair = *reinterpret_cast<const unsigned*>(h.slots + j * rows + 2 * l);
+        const unsigned a0 = pair & 0xffffu, a1 = pair >> 16;
+        at[j] = ring + a0 * kSize;
+        at[j + 1] = ring + a1 * kSize;
+        if (task.z & kFarFlag) {
+            const std::uint32_t far = smem_u32(h.far) - kFarSlot * kSize;
+            if (a0 >= kFarSlot) at[j] = far + a0 * kSize;
+            if (a1 >= kFarSlot) at[j + 1] = far + a1 * kSize;
+        }
+        coef[j] = h.coef[j * rows + l];
+        coef[j + 1] = h.coef[(j + 1) * rows + l];
+    }
+    T y = h.own[l];
+    const T fin = BACK || SSOR ? h.fin[l] : T(1);
+    if (BACK && SSOR) y = mul_rn(fin, y);
+    if (wait) bar_wait<PAIR>(wait_id);
+#pragma unroll
+    for (int j = 0; j < N; ++j) ld_ring(at[j], x[j]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) y = sub_rn(y, mul_rn(coef[j], x[j]));
+    if (SSOR) y = div_rn(y, fin);
+    else if (BACK) y = mul_rn(y, fin);
+    if (live) st_ring(slot, y);
+    if (signal) bar_signal<PAIR>(signal_id);
+    return y;
+}
+
+// The shared memory holds a stage per warp and task in flight, then the ring
+// and the slot of absent dependencies.
+// SLOW: the schedule has tasks of the slower form (a call in the loop costs
+// registers that the others need).
+template<class T, int W, int TEAMS, bool BACK, bool SSOR, bool SLOW>
+__global__ void __launch_bounds__(W * TEAMS * 32, 1) k_local_sweep(const __grid_constant__ Direction<T> d)
+{
+    constexpr int kSize = static_cast<int>(sizeof(T)), kStage = static_cast<int>(sizeof(Stage<T>));
+    constexpr int kPair = 2 * W * 32;   // threads of a barrier: the team that signals and the one that waits
+    extern __shared__ __align__(16) unsigned char shared[];
+    const int lane = threadIdx.x & 31, c = blockIdx.x;
+    const int w = threadIdx.x / 32 % W, team = threadIdx.x / (32 * W);
+    Stage<T>* const stages = reinterpret_cast<Stage<T>*>(shared) + threadIdx.x / 32 * kDepth;
+    const std::uint32_t first_stage = smem_u32(stages), ring = smem_u32(shared) + W * TEAMS * kDepth * kStage;
+    if (threadIdx.x == 0) st_ring(ring + d.ring * kSize, T(0));
+    __syncthreads();
+    const Source<T> source = source_of<T, BACK>(d, lane, c);
+    const int4* tasks = d.task + w;
+    const int* fars = d.far ? d.far + w * 32 + lane : nullptr;
+    auto task_of = [&](int s) { return s < d.steps ? __ldg(tasks + s * W) : make_int4(0, 0, 0, 0); };
+    auto far_of = [&](int s) { return fars && s < d.steps ? __ldg(fars + static_cast<std::size_t>(s) * W * 32) : -1; };
+    for (int u = 0; u < kDepth; ++u) {
+        const int4 task = task_of(team + u * TEAMS);
+        if (lane == 0) stages[u].task = task;
+        load_operands<T, BACK || SSOR>(source, lane, task, far_of(team + u * TEAMS), first_stage + u * kStage);
+    }
+    int4 next = task_of(team + kDepth * TEAMS);
+    int next_far = far_of(team + kDepth * TEAMS);
+    const int wait_id = 1 + (team + TEAMS - 1) % TEAMS, signal_id = 1 + team;
+    T* const out = d.out + (BACK ? static_cast<std::size_t>(c) : static_cast<std::size_t>(c) * d.out_places);
+    int u = 0;
+    for (int s = team; s < d.steps; s += TEAMS) {
+        Stage<T>& h = stages[u];
+        asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+        __syncwarp();
+        const int4 task = h.task;
+        const int rows = task.z & 0xff;
+        const int place = task.w + lane;
+        const std::uint32_t slot = ring + (place >= d.ring ? place - d.ring : place) * kSize;
+        const bool wait = s > 0, signal = s + 1 < d.steps;
+        T y = T(0);
+        if (rows == 0) {
+            if (wait) bar_wait<kPair>(wait_id);
+            if (signal) bar_signal<kPair>(signal_id);
+        } else if (SLOW && (task.z & kSlowFlag)) {
+            y = h.own[min(lane, rows - 1)];
+            const T fin = BACK || SSOR ? h.fin[min(lane, rows - 1)] : T(1);
+            if (BACK && SSOR) y = mul_rn(fin, y);
+            if (wait) bar_wait<kPair>(wait_id);
+            y = consume_slow<T, BACK>(y, &d, lane, c, task, ring);
+            if (SSOR) y = div_rn(y, fin);
+            else if (BACK) y = mul_rn(y, fin);
+            if (lane < rows) st_ring(slot, y);
+            if (signal) bar_signal<kPair>(signal_id);
+        } else {
+            auto run = [&](auto n) {
+                y = run_task<T, decltype(n)::value, kPair, BACK, SSOR>(h, task, lane, ring, slot, wait, signal, wait_id,
+                                                                       signal_id);
+            };
+            const int width = task.z >> 8 & 0xff;
+            if (width == 4) run(std::integral_constant<int, 4>());
+            else if (width == 6) run(std::integral_constant<int, 6>());
+            else if (width == 2) run(std::integral_constant<int, 2>());
+            else if (width == 0) run(std::integral_constant<int, 0>());
+            else run(std::integral_constant<int, 8>());
+        }
+        const int to = rows > 0 ? h.to[min(lane, rows - 1)] : 0;
+        if (lane < rows) {
+            if (y != y) y = Bits<T>::quiet_nan();
+            out[BACK ? static_cast<std::size_t>(to) * d.bs : static_cast<std::size_t>(to)] = y;
+        }
+        __syncwarp();
+        if (lane == 0) h.task = next;
+        load_operands<T, BACK || SSOR>(source, lane, next, next_far, first_stage + u * kStage);
+        next = task_of(s + (kDepth + 1) * TEAMS);
+        next_far = far_of(s + (kDepth + 1) * TEAMS);
+        u = u + 1 == kDepth ? 0 : u + 1;
+    }
+}
+
+template<class T> __device__ __forceinline__ T widen(double v) { return static_cast<T>(v); }
+template<class T> __device__ __forceinline__ T widen(float v) { return static_cast<T>(v); }
+template<class T> __device__ __forceinline__ T widen(__nv_bfloat16 v) { return static_cast<T>(__bfloat162float(v)); }
+
+// Into the sweep's layout (component-major, order of the steps): coefficients
+// and diagonals of both directions, and the right-hand side.  One thread per
+// entry or row, reading its bs values side by side; SCALE: coefficients times
+// omega (SSOR).
+template<class T, class F>
+struct PackArgs {
+    const int* src[2];
+    T* coef[2];
+    std::size_t entries[2];
+    const int* rows[2];  // per place (-1: padding)
+    T* fin[2];           // null: none
+    const T* in;         // null: none
+    T* in_to;
+    std::size_t places[2];
+    const F* vals;
+    const F* diag;
+    T omega;
+    int bs;
+};
+
+template<class T, class F, bool SCALE>
+__global__ void __launch_bounds__(kThreads) k_local_pack(PackArgs<T, F> a)
+{
+    std::size_t i = static_cast<std::size_t>(blockIdx.x) * kThreads + threadIdx.x;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        if (i < a.entries[s]) {
+            const int e = a.src[s][i];
+            if (e < 0) return;
+            for (int c = 0; c < a.bs; ++c) {
+                const T v = widen<T>(a.vals[static_cast<std::size_t>(e) * a.bs + c]);
+                a.coef[s][static_cast<std::size_t>(c) * a.entries[s] + i] = SCALE ? mul_rn(a.omega, v) : v;
+            }
+            return;
+        }
+        i -= a.entries[s];
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        if (a.fin[s] == nullptr) continue;
+        if (i < a.places[s]) {
+            const int row = a.rows[s][i];
+            if (row < 0) return;
+            for (int c = 0; c < a.bs; ++c)
+                a.fin[s][static_cast<std::size_t>(c) * a.places[s] + i] =
+                    widen<T>(a.diag[static_cast<std::size_t>(row) * a.bs + c]);
+            return;
+        }
+        i -= a.places[s];
+    }
+    if (a.in != nullptr && i < a.places[0]) {
+        const int row = a.rows[0][i];
+        if (row < 0) return;
+        for (int c = 0; c < a.bs; ++c)
+            a.in_to[static_cast<std::size_t>(c) * a.places[0] + i] = a.in[static_cast<std::size_t>(row) * a.bs + c];
+    }
+}
+
+// values / in: null leaves the coefficients and diagonals, or the right-hand side, as they are.
+template<class T, class F>
+void pack(Context& c, Preconditioner& p, const F* values, const F* diag, const T* in, T omega, bool ssor)
+{
+    PackArgs<T, F> a{};
+    LocalSweep* s[2] = {&p.lower_local, &p.upper_local};
+    std::size_t total = in ? p.lower_local.places : 0;
+    for (int k = 0; k < 2; ++k) {
+        a.places[k] = s[k]->places;
+        a.rows[k] = s[k]->rows.as<int>();
+        if (values == nullptr) continue;
+        a.src[k] = s[k]->src.as<int>();
+        a.coef[k] = s[k]->coef.as<T>();
+        a.entries[k] = s[k]->entries;
+        a.fin[k] = ssor || k == 1 ? s[k]->fin.as<T>() : nullptr;
+        total += s[k]->entries + (a.fin[k] ? s[k]->places : 0);
+    }
+    a.in = in;
+    a.in_to = p.lower_local.in.as<T>();
+    a.vals = values;
+    a.diag = diag;
+    a.omega = omega;
+    a.bs = static_cast<int>(p.bs);
+    const unsigned blocks = static_cast<unsigned>((total + kThreads - 1) / kThreads);
+    if (ssor) k_local_pack<T, F, true><<<blocks, kThreads, 0, c.stream>>>(a);
+    else k_local_pack<T, F, false><<<blocks, kThreads, 0, c.stream>>>(a);
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+}
+
+template<class T, int W, int TEAMS, bool BACK, bool SSOR>
+void launch_shape(Context& c, const Direction<T>& d)
+{
+    auto* kernel = d.code ? k_local_sweep<T, W, TEAMS, BACK, SSOR, true> : k_local_sweep<T, W, TEAMS, BACK, SSOR, false>;
+    const int bytes = W * TEAMS * kDepth * static_cast<int>(sizeof(Stage<T>)) + (d.ring + 1) * static_cast<int>(sizeof(T));
+    OWTK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes));
+    kernel<<<static_cast<unsigned>(d.bs), W * TEAMS * 32, bytes, c.stream>>>(d);
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+}
+
+template<class T, bool BACK, bool SSOR>
+void launch(Context& c, Preconditioner& p, T* out)
+{
+    const LocalSweep& s = BACK ? p.upper_local : p.lower_local;
+    Direction<T> d{};
+    d.task = s.task.as<int4>();
+    d.slots = s.slots.as<std::uint16_t>();
+    d.far = s.far.ptr ? s.far.as<int>() : nullptr;
+    d.code = s.code.ptr ? s.code.as<int>() : nullptr;
+    d.to = BACK ? s.rows.as<int>() : s.to.as<int>();
+    d.coef = s.coef.as<T>();
+    d.fin = s.fin.as<T>();
+    d.in = s.in.as<T>();
+    d.out = BACK ? out : p.upper_local.in.as<T>();
+    d.entries = s.entries;
+    d.places = s.places;
+    d.out_places = p.upper_local.places;
+    d.steps = s.steps;
+    d.ring = s.ring;
+    d.bs = static_cast<int>(p.bs);
+    switch (s.warps) {
+    case 1: launch_shape<T, 1, kTeams1, BACK, SSOR>(c, d); break;
+    case 2: launch_shape<T, 2, kTeams2, BACK, SSOR>(c, d); break;
+    default: launch_shape<T, 4, kTeams4, BACK, SSOR>(c, d); break;
+    }
+}
+
+// A direction's rows in step order, padded: each task starts at a multiple of
+// four places.
+struct Cut {
+    std::vector<std::int32_t> task;    // per step and warp: first entry, first place, rows and width, first ring slot
+    std::vector<std::int32_t> rows;    // per place (-1: padding)
+    std::vector<std::int32_t> place;   // per row
+    std::vector<std::int32_t> count;   // dependencies per row
+};
+
+// Rows by level and row number, cut into tasks and steps.  (Within a level by
+// number of dependencies, for less padding: the same times.)  False for a row
+// of more dependencies than a task's width holds.
+bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32_t* begin, const std::int32_t* end,
+               const std::int32_t* cols, bool backward, int warps)
+{
+    const auto n = static_cast<std::int32_t>(owned);
+    cut.count.assign(owned, 0);
+    for (std::int32_t r = 0; r < n; ++r)
+        for (std::int32_t e = begin[r]; e < end[r]; ++e)
+            cut.count[r] += backward ? cols[e] > r && cols[e] < n : cols[e] < r;
+    const std::vector<std::int32_t>&order = sweep.h_order, &level = sweep.h_level;
+    cut.place.resize(owned);
+    std::int32_t at = 0;
+    for (std::int32_t b = 0; b < n;) {
+        std::int32_t e = b;
+        while (e < n && level[order[e]] == level[order[b]]) ++e;
+        while (b < e) {
+            for (int w = 0; w < warps; ++w) {
+                // As many rows as their padded entries leave room for in a stage.
+                std::int32_t rows = 0, width = 0;
+                while (rows < 32 && b + rows < e) {
+                    const std::int32_t wider = std::max(width, (cut.count[order[b + rows]] + 1) / 2 * 2);
+                    if (rows > 0 && (rows + 1) * wider > kTaskEntries) break;
+                    width = wider;
+                    ++rows;
+                }
+                if (width > 0xff) return false;
+                cut.task.insert(cut.task.end(), {0, at, rows | width << 8, 0});
+                for (std::int32_t l = 0; l < rows; ++l) {
+                    cut.place[order[b + l]] = at + l;
+                    cut.rows.push_back(order[b + l]);
+                }
+                while (cut.rows.size() % 4 != 0) cut.rows.push_back(-1);
+                at = static_cast<std::int32_t>(cut.rows.size());
+                b += rows;
+            }
+        }
+    }
+    cut.rows.resize(cut.rows.size() + 32, -1);   // a task's copies always take 32 places
+    return true;
+}
+
+bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t bs, std::size_t element_size,
+                     const Sweep& sweep, Cut& cut, const Cut& other, const std::int32_t* begin, const std::int32_t* end, const std::int32_t* cols,
+                     bool backward, bool with_fin, int warps, int shared_rows)
+{
+    const auto n = static_cast<std::int32_t>(owned);
+    const std::vector<std::int32_t>& place = cut.place;
+    s.warps = warps;
+    s.places = cut.rows.size();
+    s.steps = static_cast<int>(cut.task.size() / 4) / warps;
+    s.ring = std::min(static_cast<std::int32_t>(s.places), std::min(shared_rows, kFarSlot - 1));
+    // A step's results may not overwrite what the same step still reads.
+    const std::int32_t reach = static_cast<std::int32_t>(s.places) > s.ring ? s.ring - 32 * warps : s.ring;
+    auto needed = [&](std::int32_t row, std::int32_t col) { return backward ? col > row && col < n : col < row; };
+    auto far_index = [&](std::int32_t col) { return backward ? col : other.place[col]; };
+    std::size_t first = 0, used = 0, slow_tasks = 0;
+    std::vector<std::int32_t> far;
+    for (std::size_t t = 0; t < cut.task.size(); t += 4) {
+        std::int32_t* w = cut.task.data() + t;
+        const std::int32_t rows = w[2] & 0xff, width = w[2] >> 8;
+        std::size_t found = 0;
+        for (std::int32_t p = w[1]; p < w[1] + rows; ++p) {
+            const std::int32_t row = cut.rows[p];
+            used += static_cast<std::size_t>(cut.count[row]);
+            for (std::int32_t k = begin[row]; k < end[row]; ++k) {
+                if (!needed(row, cols[k]) || p - place[cols[k]] <= reach) continue;
+                if (far.empty()) far.assign(cut.task.size() / 4 * 32, -1);
+                if (found < 32) far[t / 4 * 32 + found] = far_index(cols[k]);
+                ++found;
+            }
+        }
+        const bool slow = width > kHold || found > 32;
+        w[0] = static_cast<std::int32_t>(first);
+        w[2] |= slow ? kSlowFlag : found > 0 ? kFarFlag : 0;
+        w[3] = w[1] % s.ring;
+        first += (static_cast<std::size_t>(rows) * width + 7) / 8 * 8;
+        slow_tasks += slow;
+        if (first >= static_cast<std::size_t>(kMaxEntries)) return false;
+    }
+    s.entries = first;
+    // A few rows much longer than the rest would pad their tasks' other rows.
+    if (s.entries > 4 * used + 8 * owned + 4096) return false;
+    // A task of the slower form costs its step about a microsecond, more than
+    // a level of the level-scheduled sweep.
+    if (slow_tasks > static_cast<std::size_t>(sweep.depth) / 4) return false;
+    const bool any_slow = slow_tasks > 0;
+    std::vector<std::int32_t> code(any_slow ? s.entries : 0, s.ring), src(s.entries, -1);
+    std::vector<std::uint16_t> slots(s.entries, static_cast<std::uint16_t>(s.ring));
+    for (std::size_t t = 0; t < cut.task.size(); t += 4) {
+        const std::size_t base = static_cast<std::size_t>(cut.task[t]), rows = cut.task[t + 2] & 0xff;
+        std::size_t found = 0;
+        for (std::size_t l = 0; l < rows; ++l) {
+            const std::int32_t p = cut.task[t + 1] + static_cast<std::int32_t>(l), row = cut.rows[p];
+            std::size_t j = 0;
+            for (std::int32_t e = begin[row]; e < end[row]; ++e) {
+                if (!needed(row, cols[e])) continue;
+                const std::int32_t from = place[cols[e]];
+                const bool near = p - from <= reach;
+                const std::size_t slot = near ? from % s.ring : kFarSlot + found++ % 32;
+                slots[base + (j & ~std::size_t(1)) * rows + 2 * l + j % 2] = static_cast<std::uint16_t>(slot);
+                if (any_slow) code[base + j * rows + l] = near ? from % s.ring : -1 - far_index(cols[e]);
+                src[base + j * rows + l] = e;
+                ++j;
+            }
+        }
+    }
+    std::vector<std::int32_t> to;
+    if (!backward) {
+        to.assign(s.places, 0);
+        for (std::size_t p = 0; p < s.places; ++p)
+            if (cut.rows[p] >= 0) to[p] = other.place[cut.rows[p]];
+    }
+    s.task = upload(ctx.stream, cut.task);
+    s.slots = upload(ctx.stream, slots);
+    if (!far.empty()) s.far = upload(ctx.stream, far);
+    if (any_slow) s.code = upload(ctx.stream, code);
+    s.src = upload(ctx.stream, src);
+    s.rows = upload(ctx.stream, cut.rows);
+    s.to = upload(ctx.stream, to);
+    s.coef.allocate(bs * s.entries * element_size + 16);
+    OWTK_CUDA(cudaMemsetAsync(s.coef.ptr, 0, bs * s.entries * element_size, ctx.stream));   // padding: zero
+    if (with_fin) s.fin.allocate(bs * s.places * element_size + 16);
+    s.in.allocate(bs * s.places * element_size + 16);
+    s.ready = true;
+    return true;
+}
+
+constexpr int teams_of(int warps) { return warps == 1 ? kTeams1 : warps == 2 ? kTeams2 : kTeams4; }
+
+}  // namespace
+
+// Warps per team of the cheapest shape, or 0 when the level-scheduled sweep is
+// cheaper: the steps of each shape at their measured cost against 800 ns a
+// level (0.71 to 0.86 us measured at 250 to 1,400 rows a level).  The line lies
+// at about 700 rows a level, where both take 0.8 us.
+int local_sweep_warps(const Context& ctx, const Sweep& lower, const Sweep& upper, std::size_t owned, std::size_t bs)
+{
+    static constexpr struct { int warps; double ns; } kShapes[] = {{1, 75}, {2, 95}, {4, 145}};
+    const char* env = std::getenv("OWTK_LOCAL_SWEEP");   // 0: never
+    if (env && std::atoi(env) == 0) return 0;
+    if (owned == 0 || bs > static_cast<std::size_t>(ctx.sm_count)) return 0;
+    std::vector<std::size_t> size;
+    for (const Sweep* s : {&lower, &upper}) {
+        const std::size_t at = size.size();
+        size.resize(at + static_cast<std::size_t>(s->depth), 0);
+        for (std::size_t r = 0; r < owned; ++r) ++size[at + static_cast<std::size_t>(s->h_level[r])];
+    }
+    double least = 800.0 * static_cast<double>(size.size());
+    int best = 0;
+    for (const auto& k : kShapes) {
+        double cost = 0;
+        for (const std::size_t rows : size)
+            cost += static_cast<double>((rows + 32 * k.warps - 1) / (32 * k.warps)) * k.ns;
+        if (cost < least) {
+            least = cost;
+            best = k.warps;
+        }
+    }
+    return best;
+}
+
+// Dependencies of row r: entries [lower_begin[r], lower_end[r]) with a column
+// below r, and [upper_begin[r], upper_end[r]) with one above it.
+void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t element_size,
+                       const std::int32_t* lower_begin, const std::int32_t* lower_end, const std::int32_t* upper_begin,
+                       const std::int32_t* upper_end, const std::int32_t* cols, bool ssor)
+{
+    const std::size_t stage = element_size == 8 ? sizeof(Stage<double>) : sizeof(Stage<float>);
+    const int shared_rows =
+        static_cast<int>((kSharedBytes - static_cast<std::size_t>(warps * teams_of(warps) * kDepth) * stage) / element_size) - 2;
+    Cut lower, upper;
+    if (!cut_steps(lower, p.lower, p.owned, lower_begin, lower_end, cols, false, warps)
+        || !cut_steps(upper, p.upper, p.owned, upper_begin, upper_end, cols, true, warps)) return;
+    if (!build_direction(ctx, p.lower_local, p.owned, p.bs, element_size, p.lower, lower, upper, lower_begin, lower_end, cols,
+                         false, ssor, warps, shared_rows)
+        || !build_direction(ctx, p.upper_local, p.owned, p.bs, element_size, p.upper, upper, lower, upper_begin, upper_end,
+                            cols, true, true, warps, shared_rows)) {
+        p.lower_local = LocalSweep();
+        p.upper_local = LocalSweep();
+    }
+}
+
+namespace kern {
+
+template<class T, class F>
+void local_ilu_pack(Context& c, Preconditioner& p, const F* factors, const F* inverse)
+{
+    pack<T, F>(c, p, factors, inverse, nullptr, T(1), false);
+}
+
+template<class T> void local_ilu_apply(Context& c, Preconditioner& p, const T* in, T* out)
+{
+    pack<T, T>(c, p, nullptr, nullptr, in, T(1), false);
+    launch<T, false, false>(c, p, out);
+    launch<T, true, false>(c, p, out);
+}
+
+// The matrix's values are read at every apply, as the level-scheduled sweep
+// reads them: they may have been written since the last one.
+template<class T>
+void local_ssor_apply(Context& c, Preconditioner& p, const T* values, const T* diag, const T* in, T* out)
+{
+    pack<T, T>(c, p, values, diag, in, static_cast<T>(p.parameter), true);
+    launch<T, false, true>(c, p, out);
+    launch<T, true, true>(c, p, out);
+}
+
+template void local_ilu_pack<double, double>(Context&, Preconditioner&, const double*, const double*);
+template void local_ilu_pack<float, float>(Context&, Preconditioner&, const float*, const float*);
+template void local_ilu_pack<float, __nv_bfloat16>(Context&, Preconditioner&, const __nv_bfloat16*,
+                                                   const __nv_bfloat16*);
+template void local_ilu_apply<double>(Context&, Preconditioner&, const double*, double*);
+template void local_ilu_apply<float>(Context&, Preconditioner&, const float*, float*);
+template void local_ssor_apply<double>(Context&, Preconditioner&, const double*, const double*, const double*,
+                                       double*);
+template void local_ssor_apply<float>(Context&, Preconditioner&, const float*, const float*, const float*, float*);
+
+}  // namespace kern
+}  // namespace owtk

@@ -842,6 +842,8 @@ template<class T> void ilu_factorize(Context& c, Preconditioner& p, const T* mat
     for (Sweep* s : {&p.lower, &p.upper})
         if (s->packed)
             gather_values<T>(c, s->pentries, p.bs, s->psrc.as<std::int64_t>(), p.d_fvalues.as<T>(), s->pvals.as<T>());
+    if (p.upper_local.ready && p.storage == OWTK_F64)
+        local_ilu_pack<T, T>(c, p, p.d_fvalues.as<T>(), p.inv_diag.as<T>());
 }
 
 template<class T> void fill_sentinel(Context& c, std::size_t n, T* x)
@@ -859,6 +861,10 @@ template<class T> void ilu_apply(Context& c, Preconditioner& p, const T* in, T* 
     if (chain_ilu_apply<T>(c, p, in, out)) return;
     if (lockstep_ilu_apply<T>(c, p, in, out)) return;
     if (cluster_ilu_apply<T>(c, p, in, out)) return;
+    if (p.upper_local.ready) {
+        local_ilu_apply<T>(c, p, in, out);
+        return;
+    }
     SweepArgs<T> a{};
     a.rowptr = p.d_frowptr.as<int>();
     a.cols = p.d_fcols.as<int>();
@@ -889,21 +895,27 @@ template<class T> void ilu_apply(Context& c, Preconditioner& p, const T* in, T* 
 template<class T> void ssor_apply(Context& c, Preconditioner& p, const T* in, T* out)
 {
     const Matrix& m = *p.matrix;
+    const T* diag = p.kind == OWTK_PC_SPLIT_SSOR ? static_cast<const T*>(m.diag) : p.diag_cache.as<T>();
+    const T omega = static_cast<T>(p.parameter);
+    if (p.upper_local.ready) {
+        local_ssor_apply<T>(c, p, static_cast<const T*>(m.value_ptr()), diag, in, out);
+        if (omega != T(1)) scale<T>(c, p.owned * p.bs, omega * (T(2) - omega), out);
+        return;
+    }
     SweepArgs<T> a{};
     a.rowptr = m.rowptr.as<int>();
     a.cols = m.cols.as<int>();
     a.vals = const_cast<T*>(static_cast<const T*>(m.value_ptr()));
-    a.diag = p.kind == OWTK_PC_SPLIT_SSOR ? static_cast<const T*>(m.diag) : p.diag_cache.as<T>();
+    a.diag = diag;
     a.in = in;
     a.out = out;
     a.work = p.work.as<T>();
-    a.omega = static_cast<T>(p.parameter);
+    a.omega = omega;
     const std::size_t n = p.owned * p.bs;
     fill_sentinel<T>(c, n, a.work);
     launch<T, T, kSsorForward>(c, p, p.lower, a);
     fill_sentinel<T>(c, n, out);
     launch<T, T, kSsorBackward>(c, p, p.upper, a);
-    const T omega = static_cast<T>(p.parameter);
     if (omega != T(1)) scale<T>(c, p.owned * p.bs, omega * (T(2) - omega), out);
 }
 
@@ -911,6 +923,10 @@ template<class T> void ssor_apply(Context& c, Preconditioner& p, const T* in, T*
 // vectors / arithmetic: the inner preconditioner of mixed-precision solves.
 template<class F> void ilu_apply_lp(Context& c, Preconditioner& p, const float* in, float* out)
 {
+    if (p.upper_local.ready) {
+        local_ilu_apply<float>(c, p, in, out);
+        return;
+    }
     SweepArgs<float, F> a{};
     a.rowptr = p.d_frowptr.as<int>();
     a.cols = p.d_fcols.as<int>();

@@ -241,6 +241,28 @@ struct ChainSweep {
 // Rows per level (both DAGs) below which the ILU applies take the chain sweep.
 constexpr int kChainRowsPerLevel = 8;
 
+// One direction of an ILU or SSOR apply by one CTA per component
+// (kernels_local_sweep.cu): rows in step order, a step's tasks from one level;
+// a task's dependencies padded to its longest row (made even),
+// [dependency][row], its entries to 8 and its rows to 4.
+struct LocalSweep {
+    bool ready = false;
+    int steps = 0;
+    int warps = 1;             // tasks per step
+    int ring = 0;              // places whose results shared memory holds
+    std::size_t entries = 0;   // padded
+    std::size_t places = 0;    // padded rows
+    DeviceBuffer task;         // int4 per step and warp: first entry, first place, rows and width (and flags), ring slot
+    DeviceBuffer slots;        // uint16 per entry, the two of a pair side by side: ring slot or staged far value
+    DeviceBuffer far;          // 32 int32 per task, if any task has one: dependencies beyond the ring's reach
+    DeviceBuffer code;         // int32 per entry, if any task needs it: ring slot or far dependency
+    DeviceBuffer src;          // int32 per entry: factor or matrix entry (-1: padding)
+    DeviceBuffer rows;         // int32 per place: row (-1: padding)
+    DeviceBuffer to;           // int32 per place: its place in the other direction's order (forward only)
+    DeviceBuffer coef;         // per component and entry
+    DeviceBuffer fin;          // per component and place: what scales or divides the result
+    DeviceBuffer in;           // per component and place: right-hand side, or the forward result
+};
 struct Preconditioner {
     Context* ctx = nullptr;
     owtk_pc_kind kind = OWTK_PC_IDENTITY;
@@ -267,6 +289,7 @@ struct Preconditioner {
     ClusterSweep c_lower, c_upper;
     ChainSweep chain;
     LockstepSweep l_lower, l_upper;
+    LocalSweep lower_local, upper_local;
     DeviceBuffer d_floc;
     DeviceBuffer flags;        // uint32 per row, epoch-stamped
     DeviceBuffer ticket;       // uint64 monotone task counter
@@ -325,6 +348,10 @@ void build_cluster_sweep(Context& ctx, ClusterSweep& s, std::size_t owned, std::
                          const std::vector<std::int32_t>& level, const std::vector<std::int32_t>& rowptr,
                          const std::vector<std::int32_t>& cols, const std::vector<std::int32_t>& diagpos,
                          bool backward, std::vector<std::uint32_t>& loc);
+int local_sweep_warps(const Context& ctx, const Sweep& lower, const Sweep& upper, std::size_t owned, std::size_t bs);
+void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t element_size,
+                       const std::int32_t* lower_begin, const std::int32_t* lower_end, const std::int32_t* upper_begin,
+                       const std::int32_t* upper_end, const std::int32_t* cols, bool ssor);
 void rcm_order(std::size_t owned, const std::int32_t* rowptr, const std::int32_t* cols,
                std::uint64_t* out);
 void hilbert_order(std::size_t n, const double* xy, std::uint64_t* out);
@@ -409,6 +436,10 @@ template<class T> void ilu_apply(Context& c, Preconditioner& p, const T* in, T* 
 template<class T> bool cluster_ilu_apply(Context& c, Preconditioner& p, const T* in, T* out);
 template<class T> bool chain_ilu_apply(Context& c, Preconditioner& p, const T* in, T* out);
 template<class T> bool lockstep_ilu_apply(Context& c, Preconditioner& p, const T* in, T* out);
+template<class T, class F> void local_ilu_pack(Context& c, Preconditioner& p, const F* factors, const F* inverse);
+template<class T> void local_ilu_apply(Context& c, Preconditioner& p, const T* in, T* out);
+template<class T>
+void local_ssor_apply(Context& c, Preconditioner& p, const T* values, const T* diag, const T* in, T* out);
 // Test hook: a sweep whose only dependency is never published (bounded wait).
 void debug_unpublished_dependency(Context& c, int spin_limit);
 template<class T> void ssor_apply(Context& c, Preconditioner& p, const T* in, T* out);

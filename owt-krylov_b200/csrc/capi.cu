@@ -241,6 +241,7 @@ void ilu_symbolic(Preconditioner& p, const Matrix& m, std::size_t fill)
     p.d_upd_start = upload(s, start);
     p.d_upd_target = upload(s, target);
     p.d_upd_upper = upload(s, upper);
+    kern::build_factor_programs(*p.ctx, p);
     const std::size_t per = p.block ? p.bs * p.bs : p.bs;   // values per factor entry
     p.d_fvalues.allocate(nnz * per * dsize(p.dtype) + 16);
     p.inv_diag.allocate(n * per * dsize(p.dtype) + 16);

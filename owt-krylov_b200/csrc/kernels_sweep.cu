@@ -32,6 +32,7 @@
 // in entry order, with explicit rounding (device_common.cuh), so results equal
 // the CPU path bit for bit whatever order the rows complete in.
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdlib>
@@ -770,6 +771,138 @@ __global__ void __launch_bounds__(kThreads) k_sweep(SweepArgs<T, F> a)
     }
 }
 
+// Numeric ILU factorisation synchronised on the data, like the applies: the
+// factor values are first filled with the sentinel, a row polls for the pivots
+// and upper entries that its elimination reads and publishes its diagonal and
+// upper entries.  Half a warp holds one (row, component), an entry per lane, so
+// the subtractions of one pivot step run side by side and a level costs one L2
+// hand-off plus a division and a shuffle per lower entry; indices and matrix
+// values are loaded, and all operands polled at once, before the first step.
+// For rows of up to 16 entries and 8 lower ones; others keep per-row flags
+// (row_body), behind which the values are read one by one.  50,000 rows, bs 4,
+// 871 levels: 11.1 ms with the flags, 3.3 ms with one lane per (row, component)
+// and the row in shared memory, 1.7 ms so.
+constexpr int kFactorRow = 16;        // lanes of a (row, component)
+constexpr int kFactorLower = 8;
+
+// Per row and lower entry l, for each of the row's entries e: the factor entry
+// that step l multiplies for e (the pivot's upper entry of the same column), or
+// -1; at e = l, the pivot.
+__global__ void __launch_bounds__(kThreads) k_factor_program(int n, const int* rowptr, const int* diagpos,
+                                                             const int* cols, const int* upd_start,
+                                                             const int* upd_target, const int* upd_upper,
+                                                             const int* start, int* program)
+{
+    const int row = blockIdx.x * kThreads + threadIdx.x;
+    if (row >= n) return;
+    const int b = rowptr[row], d = diagpos[row], len = rowptr[row + 1] - b;
+    for (int l = b; l < d; ++l) {
+        int* step = program + start[row] + (l - b) * len;
+        for (int e = 0; e < len; ++e) step[e] = -1;
+        step[l - b] = diagpos[cols[l]];
+        for (int u = upd_start[l]; u < upd_start[l + 1]; ++u) step[upd_target[u] - b] = upd_upper[u];
+    }
+}
+
+template<class T>
+struct FactorArgs {
+    const int* order;
+    int owned;
+    const int* rowptr;
+    const int* diagpos;
+    const int* start;             // program of each row
+    const int* program;
+    const std::int64_t* source;   // matrix entry of each factor entry, or -1
+    const T* matrix;
+    T* vals;
+    T* inv;
+    int bs;
+    unsigned long long* ticket;
+    unsigned long long base;
+    unsigned* status;
+};
+
+template<class T>
+__global__ void __launch_bounds__(kThreads) k_ilu_factor(FactorArgs<T> a)
+{
+    using U = typename Bits<T>::U;
+    const int lane = threadIdx.x & 31, e = lane % kFactorRow, half = lane / kFactorRow, bs = a.bs;
+    const unsigned per_row = static_cast<unsigned>((bs + 1) / 2);   // warp tasks per row: two components each
+    const unsigned long long tasks = static_cast<unsigned long long>(a.owned) * per_row;
+    const T tol = pivot_tolerance<T>();
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(a.ticket, 1ull) - a.base;
+    for (;;) {
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= tasks) break;
+        unsigned long long next = 0;
+        if (lane == 0) next = atomicAdd(a.ticket, 1ull) - a.base;
+        const unsigned q = static_cast<unsigned>(t / per_row);
+        const int c = static_cast<int>(t - static_cast<unsigned long long>(q) * per_row) * 2 + half;
+        const int row = a.order[q];
+        const int b = a.rowptr[row], lower = a.diagpos[row] - b, len = a.rowptr[row + 1] - b, p0 = a.start[row];
+        const bool live = c < bs && e < len;
+        T v = T(0);
+        int need[kFactorLower];
+#pragma unroll
+        for (int l = 0; l < kFactorLower; ++l) need[l] = live && l < lower ? a.program[p0 + l * len + e] : -1;
+        if (live) {
+            const std::int64_t from = a.source[b + e];
+            if (from >= 0) v = a.matrix[from * bs + c];
+        }
+        U x[kFactorLower];
+#pragma unroll
+        for (int l = 0; l < kFactorLower; ++l) {
+            x[l] = U(0);
+            if (need[l] >= 0) x[l] = ld_relaxed_bits(a.vals + static_cast<std::size_t>(need[l]) * bs + c);
+        }
+        for (int it = 0;; ++it) {
+            bool pending = false;
+#pragma unroll
+            for (int l = 0; l < kFactorLower; ++l) pending |= x[l] == Bits<T>::kSentinel;
+            if (!__any_sync(0xffffffffu, pending)) break;
+            if (it >= kSpinLimit) {
+                if (lane == 0) atomicOr(a.status, kErrTimeout);
+                break;
+            }
+            if ((it & 1023) == 1023
+                && __any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned*>(a.status) & kErrTimeout)) break;
+            if (it >= 256) __nanosleep(32);
+#pragma unroll
+            for (int l = 0; l < kFactorLower; ++l)
+                if (x[l] == Bits<T>::kSentinel)
+                    x[l] = ld_relaxed_bits(a.vals + static_cast<std::size_t>(need[l]) * bs + c);
+        }
+        // Step l: lane l divides by its pivot, the lanes of the columns that
+        // the pivot row has too subtract.
+#pragma unroll
+        for (int l = 0; l < kFactorLower; ++l) {
+            if (l < lower) {
+                if (live && e == l) {
+                    const T piv = from_bits(x[l]);
+                    if (fabs(piv) <= tol) atomicOr(a.status, kErrZeroPivot);
+                    v = div_rn(v, piv);
+                }
+                const T lv = __shfl_sync(0xffffffffu, v, half * kFactorRow + l);
+                if (e != l && need[l] >= 0) v = sub_rn(v, mul_rn(lv, from_bits(x[l])));
+            }
+        }
+        if (live) {
+            T* dst = a.vals + static_cast<std::size_t>(b + e) * bs + c;
+            if (e < lower) {
+                *dst = v;
+            } else {
+                publish(dst, v);
+                if (e == lower) {
+                    if (!isfinite(v) || fabs(v) <= tol) atomicOr(a.status, kErrZeroPivot);
+                    a.inv[static_cast<std::size_t>(row) * bs + c] = div_rn(T(1), v);
+                }
+            }
+        }
+        t = next;
+    }
+}
+
 // Warps per sweep launch: enough to hold a few levels' worth of tasks in
 // flight.  More warps only add polling traffic on the dependency flags while
 // the sweep is bound by its level-to-level latency.
@@ -825,7 +958,73 @@ void launch(Context& c, Preconditioner& p, Sweep& s, SweepArgs<T, F>& a)
 
 namespace kern {
 
-template<class T> void ilu_factorize(Context& c, Preconditioner& p, const T* matrix_values)
+template<class T> void fill_sentinel(Context& c, std::size_t n, T* x)
+{
+    if (n == 0) return;
+    k_fill_sentinel<T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, c.stream>>>(n, x);
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+}
+
+// The programs of k_ilu_factor, for component-diagonal factors whose rows fit.
+void build_factor_programs(Context& c, Preconditioner& p)
+{
+    if (p.block) return;
+    const std::size_t n = p.owned;
+    std::vector<std::int32_t> start(n + 1, 0);
+    std::int64_t total = 0;
+    for (std::size_t r = 0; r < n; ++r) {
+        const std::int32_t lower = p.f_diagpos[r] - p.f_rowptr[r], len = p.f_rowptr[r + 1] - p.f_rowptr[r];
+        if (len > kFactorRow || lower > kFactorLower) return;
+        total += lower * len;
+        if (total >= INT32_MAX) return;
+        start[r + 1] = static_cast<std::int32_t>(total);
+    }
+    p.d_prog_start = upload(c.stream, start);
+    p.d_program.allocate(static_cast<std::size_t>(total) * 4 + 16);
+    k_factor_program<<<static_cast<unsigned>((n + kThreads - 1) / kThreads), kThreads, 0, c.stream>>>(
+        static_cast<int>(n), p.d_frowptr.as<int>(), p.d_fdiagpos.as<int>(), p.d_fcols.as<int>(), p.d_upd_start.as<int>(),
+        p.d_upd_target.as<int>(), p.d_upd_upper.as<int>(), p.d_prog_start.as<int>(), p.d_program.as<int>());
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+}
+
+namespace {
+
+// The factorisation in k_ilu_factor; false where its rows do not fit.
+template<class T> bool factor_by_data(Context& c, Preconditioner& p, const T* matrix_values)
+{
+    if (!p.d_prog_start.ptr) return false;
+    const Sweep& s = p.lower;
+    fill_sentinel<T>(c, p.f_cols.size() * p.bs, p.d_fvalues.as<T>());
+    FactorArgs<T> a{};
+    a.order = s.order.as<int>();
+    a.owned = static_cast<int>(p.owned);
+    a.rowptr = p.d_frowptr.as<int>();
+    a.diagpos = p.d_fdiagpos.as<int>();
+    a.start = p.d_prog_start.as<int>();
+    a.program = p.d_program.as<int>();
+    a.source = p.d_fsource.as<std::int64_t>();
+    a.matrix = matrix_values;
+    a.vals = p.d_fvalues.as<T>();
+    a.inv = p.inv_diag.as<T>();
+    a.bs = static_cast<int>(p.bs);
+    a.ticket = p.ticket.as<unsigned long long>();
+    a.base = p.ticket_base;
+    a.status = c.status.as<unsigned>();
+    // Warps for sixteen levels, so that a row's own loads are over when its
+    // dependencies arrive.
+    const std::size_t tasks = p.owned * ((p.bs + 1) / 2), per_level = (tasks + s.depth - 1) / s.depth;
+    const std::size_t warps = std::min({tasks, 16 * per_level, static_cast<std::size_t>(c.sm_count) * 32});
+    const int per_block = kThreads / 32, blocks = static_cast<int>((warps + per_block - 1) / per_block);
+    k_ilu_factor<T><<<blocks, kThreads, 0, c.stream>>>(a);
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+    p.ticket_base += tasks + static_cast<unsigned long long>(blocks) * per_block;
+    return true;
+}
+
+template<class T> void factor_by_flags(Context& c, Preconditioner& p, const T* matrix_values)
 {
     gather_values<T>(c, p.f_cols.size(), p.bs, p.d_fsource.as<std::int64_t>(), matrix_values,
                      p.d_fvalues.as<T>());
@@ -839,19 +1038,18 @@ template<class T> void ilu_factorize(Context& c, Preconditioner& p, const T* mat
     a.upd_target = p.d_upd_target.as<int>();
     a.upd_upper = p.d_upd_upper.as<int>();
     launch<T, T, kIluFactor>(c, p, p.lower, a);
+}
+
+}  // namespace
+
+template<class T> void ilu_factorize(Context& c, Preconditioner& p, const T* matrix_values)
+{
+    if (!factor_by_data<T>(c, p, matrix_values)) factor_by_flags<T>(c, p, matrix_values);
     for (Sweep* s : {&p.lower, &p.upper})
         if (s->packed)
             gather_values<T>(c, s->pentries, p.bs, s->psrc.as<std::int64_t>(), p.d_fvalues.as<T>(), s->pvals.as<T>());
     if (p.upper_local.ready && p.storage == OWTK_F64)
         local_ilu_pack<T, T>(c, p, p.d_fvalues.as<T>(), p.inv_diag.as<T>());
-}
-
-template<class T> void fill_sentinel(Context& c, std::size_t n, T* x)
-{
-    if (n == 0) return;
-    k_fill_sentinel<T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, c.stream>>>(n, x);
-    OWTK_CUDA(cudaGetLastError());
-    c.launched();
 }
 
 // preconditioner.hpp:320-363.  The forward result goes to the PC's work

@@ -282,6 +282,8 @@ struct Preconditioner {
     // IKJ update list of the numeric factorisation: for every lower entry l,
     // the (target, upper) entry pairs it updates, in reference order.
     DeviceBuffer d_upd_start, d_upd_target, d_upd_upper;
+    // The same as one program per row (kernels_sweep.cu), where the rows fit.
+    DeviceBuffer d_prog_start, d_program;
     // SSOR dependency patterns reuse the matrix structure.
     Sweep lower, upper;
     // Cluster schedules of the ILU applies and, per factor entry, where its
@@ -431,6 +433,7 @@ void slices_fill(Context& c, Matrix& m);
 template<class T> void gather_values(Context& c, std::size_t entries, std::size_t bs,
                                      const std::int64_t* source, const T* values, T* out);
 // ILU(0)/SSOR sweeps.
+void build_factor_programs(Context& c, Preconditioner& p);
 template<class T> void ilu_factorize(Context& c, Preconditioner& p, const T* matrix_values);
 template<class T> void ilu_apply(Context& c, Preconditioner& p, const T* in, T* out);
 template<class T> bool cluster_ilu_apply(Context& c, Preconditioner& p, const T* in, T* out);

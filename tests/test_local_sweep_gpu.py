@@ -158,3 +158,27 @@ def test_fp32_equals_level_scheduled(native, ctx, problems, monkeypatch, kind):
     local.apply(xv, y1)
     levels.apply(xv, y2)
     assert_bitwise(y1.download(), y2.download(), kind)
+
+
+@pytest.mark.parametrize("bs,lower", [(1, 3), (2, 8), (3, 9), (5, 5), (33, 4)])
+def test_factors(native, ctx, restatement, bs, lower):
+    # The data-synchronised factorisation takes rows of up to 16 entries and 8
+    # lower ones; both sides of that line, odd and large block sizes.
+    n, rp, ci, v = _rows_system(900, bs, lower, lambda r, g: [r - 1, r - 2, *range(r - 20, r - 20 - (lower - 2), -1)])
+    m = native.Matrix(ctx, "bsr", n, 0, bs, rp, ci, v)
+    p = native.Preconditioner(m, native.PC_ILU, 0)
+    _, _, vals, inv = p.ilu_factors()
+    want = restatement.ilu(n, bs, rp, ci, v, 0).factors()
+    assert_bitwise(vals, want[2], "factors")
+    assert_bitwise(inv, want[3], "inverse diagonal")
+
+
+def test_factor_zero_pivot(native, ctx, problems):
+    n, rp, ci, v = _lattice(problems, 30, 20, 2, 6)
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    v = v.reshape(-1, 2).copy()
+    v[(ci == rows) & (rows == 0)] = 0.0
+    m = native.Matrix(ctx, "bsr", n, 0, 2, rp, ci, v.reshape(-1))
+    with pytest.raises(native.OwtkError) as err:
+        native.Preconditioner(m, native.PC_ILU, 0)
+    assert err.value.kind == "zero_pivot"

@@ -1140,6 +1140,7 @@ __global__ void __launch_bounds__(256) k_gnn_out_grad(long long count, const flo
         red[1][threadIdx.x >> 5] = acc_r;
     }
     __syncthreads();
+    __shared__ bool last;
     if (threadIdx.x == 0) {
         double be = 0.0, br = 0.0;
         for (int w = 0; w < 8; ++w) {
@@ -1149,16 +1150,23 @@ __global__ void __launch_bounds__(256) k_gnn_out_grad(long long count, const flo
         partials[2 * blockIdx.x] = be;
         partials[2 * blockIdx.x + 1] = br;
         __threadfence();
-        if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
-            __threadfence();
-            double te = 0.0, tr = 0.0;
-            for (unsigned k = 0; k < gridDim.x; ++k) {
-                te += __ldcg(partials + 2 * k);
-                tr += __ldcg(partials + 2 * k + 1);
-            }
-            *loss = (ee > 0.0 ? we * te / ee : 0.0) + (rr > 0.0 ? wr * tr / rr : 0.0);
-            *ticket = 0;
-        }
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    // The last block's first warp: lane k takes blocks k, k + 32, ... (one
+    // thread walking all 512 took two thirds of the kernel's 31 us).
+    __threadfence();
+    double te = 0.0, tr = 0.0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += 32) {
+        te += __ldcg(partials + 2 * k);
+        tr += __ldcg(partials + 2 * k + 1);
+    }
+    te = warp_sum(te);
+    tr = warp_sum(tr);
+    if (threadIdx.x == 0) {
+        *loss = (ee > 0.0 ? we * te / ee : 0.0) + (rr > 0.0 ? wr * tr / rr : 0.0);
+        *ticket = 0;
     }
 }
 
@@ -1169,59 +1177,117 @@ __global__ void k_gnn_residual(long long count, const double* __restrict__ r, co
     if (i < count) res[i] = static_cast<float>(r[i] - static_cast<double>(ax[i]));
 }
 
-// dh4 = dz Wd (FP32 rows of 64).
+// dh4 = dz Wd (FP32 rows of 64): 16 lanes per vertex, 4 features each, so a
+// row leaves as one coalesced run (a thread per vertex, each writing its row,
+// took 56 us for 100,000 vertices).
 __global__ void __launch_bounds__(256) k_gnn_decode_bwd(int n, int bs, const float* __restrict__ dz,
                                                         const float* __restrict__ wd, float* __restrict__ dh)
 {
     __shared__ float w[8 * kH];
     for (int i = threadIdx.x; i < 8 * kH; i += blockDim.x) w[i] = wd[i];
     __syncthreads();
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int v = static_cast<int>(t >> 4), k4 = static_cast<int>(t & 15);
     if (v >= n) return;
-    float d[8];
-    for (int c = 0; c < 8; ++c) d[c] = c < bs ? dz[static_cast<long long>(v) * bs + c] : 0.0f;
-    float4* o = reinterpret_cast<float4*>(dh + static_cast<long long>(v) * kH);
+    float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int c = 0; c < bs; ++c) {
+        const float d = dz[static_cast<long long>(v) * bs + c];
 #pragma unroll
-    for (int k4 = 0; k4 < kH / 4; ++k4) {
-        float r[4];
+        for (int i = 0; i < 4; ++i) r[i] = fmaf(d, w[c * kH + k4 * 4 + i], r[i]);
+    }
+    reinterpret_cast<float4*>(dh + static_cast<long long>(v) * kH)[k4] = make_float4(r[0], r[1], r[2], r[3]);
+}
+
+// Per-block partials of G[i][j] = sum_v a[v][i] * b[v][j] (a: FP32 rows of PA,
+// b: rows of PB in BF16 or FP32), PA * PB <= 1024; rows split into contiguous
+// block ranges, summed in row order.  The rows pass through shared memory in
+// coalesced chunks: 64 x 16 over 100,000 rows 317 -> 36 us, 3 x 64 159 ->
+// 20 us, against one sum per thread and pass with both factors read from
+// global memory.
+constexpr int kOuterRows = 64;
+
+// count consecutive values at src into shared memory as floats; eight loads a
+// thread in flight.
+template<class B>
+__device__ __forceinline__ void stage_rows(float* dst, const B* __restrict__ src, int count)
+{
+    constexpr int kPer = 16 / static_cast<int>(sizeof(B));
+    if (count % kPer == 0 && reinterpret_cast<std::uintptr_t>(src) % 16 == 0) {
+#pragma unroll 8
+        for (int k = threadIdx.x; k < count / kPer; k += 256) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(src) + k);
+            const B* x = reinterpret_cast<const B*>(&u);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float acc = 0.0f;
-            for (int c = 0; c < bs; ++c) acc = fmaf(d[c], w[c * kH + k4 * 4 + i], acc);
-            r[i] = acc;
+            for (int i = 0; i < kPer; i += 4)
+                *reinterpret_cast<float4*>(dst + k * kPer + i) =
+                    make_float4(static_cast<float>(x[i]), static_cast<float>(x[i + 1]), static_cast<float>(x[i + 2]),
+                                static_cast<float>(x[i + 3]));
         }
-        o[k4] = make_float4(r[0], r[1], r[2], r[3]);
+    } else {
+#pragma unroll 8
+        for (int k = threadIdx.x; k < count; k += 256) dst[k] = static_cast<float>(src[k]);
     }
 }
 
-// Per-block partials of G[i][j] = sum_v a[v][i] * b[v][j] (a: FP32 rows of pa,
-// b: rows of pb in BF16 or FP32), i < pa, j < pb, pa * pb <= 1024; rows split
-// into contiguous block ranges, summed in row order.
+// A thread sums four neighbouring columns of one row of G: one broadcast and
+// one 16-byte shared load for four FMAs.
 template<class B>
 __global__ void __launch_bounds__(256) k_gnn_outer(int n, int pa, int pb, const float* __restrict__ a,
                                                    const B* __restrict__ b, float* __restrict__ partials)
 {
+    __shared__ __align__(16) float sa[kOuterRows * kH], sb[kOuterRows * kH];   // pa, pb <= 64; pb a multiple of 4
     const int rows = (n + gridDim.x - 1) / gridDim.x;
     const int v0 = blockIdx.x * rows, v1 = min(n, v0 + rows);
-    for (int t = threadIdx.x; t < pa * pb; t += blockDim.x) {
-        const int i = t / pb, j = t - i * pb;
-        float acc = 0.0f;
-        for (int v = v0; v < v1; ++v)
-            acc = fmaf(a[static_cast<long long>(v) * pa + i], static_cast<float>(b[static_cast<long long>(v) * pb + j]),
-                       acc);
-        partials[static_cast<long long>(blockIdx.x) * pa * pb + t] = acc;
+    const int i = threadIdx.x / (pb / 4), j = threadIdx.x % (pb / 4) * 4;
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int r0 = v0; r0 < v1; r0 += kOuterRows) {
+        const int m = min(kOuterRows, v1 - r0);
+        __syncthreads();
+        stage_rows(sa, a + static_cast<long long>(r0) * pa, m * pa);
+        stage_rows(sb, b + static_cast<long long>(r0) * pb, m * pb);
+        __syncthreads();
+        if (i < pa) {
+#pragma unroll 8
+            for (int r = 0; r < m; ++r) {
+                const float x = sa[r * pa + i];
+                const float4 y = *reinterpret_cast<const float4*>(sb + r * pb + j);
+                acc.x = fmaf(x, y.x, acc.x);
+                acc.y = fmaf(x, y.y, acc.y);
+                acc.z = fmaf(x, y.z, acc.z);
+                acc.w = fmaf(x, y.w, acc.w);
+            }
+        }
     }
+    if (i < pa)
+        *reinterpret_cast<float4*>(partials + static_cast<long long>(blockIdx.x) * pa * pb + i * pb + j) = acc;
 }
 
-// Sum `blocks` partial arrays of `count` floats in block order into out[]
-// (optionally transposed: out[j * rows + i] for element i * cols + j).
-__global__ void k_gnn_reduce(int blocks, int count, const float* __restrict__ partials, float* __restrict__ out,
-                             int rows, int cols, int transpose)
+// Sum `blocks` partial arrays of `count` floats into out[] (optionally
+// transposed: out[j * rows + i] for element i * cols + j): a block takes 32
+// elements, each of its warps a run of the partial arrays in order, and the
+// runs are added in order.
+constexpr int kReduceWarps = 8;
+
+__global__ void __launch_bounds__(kReduceWarps * 32) k_gnn_reduce(int blocks, int count,
+                                                                  const float* __restrict__ partials,
+                                                                  float* __restrict__ out, int rows, int cols,
+                                                                  int transpose)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
+    __shared__ float runs[kReduceWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = blockIdx.x * 32 + lane;
+    const int per = (blocks + kReduceWarps - 1) / kReduceWarps;
     float acc = 0.0f;
-    for (int b = 0; b < blocks; ++b) acc += partials[static_cast<long long>(b) * count + t];
+    if (t < count) {
+        const int end = min(blocks, (w + 1) * per);
+#pragma unroll 16
+        for (int b = w * per; b < end; ++b) acc += __ldg(partials + static_cast<long long>(b) * count + t);
+    }
+    runs[w][lane] = acc;
+    __syncthreads();
+    if (w != 0 || t >= count) return;
+    acc = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kReduceWarps; ++k) acc += runs[k][lane];
     if (transpose) {
         const int i = t / cols, j = t - i * cols;
         out[j * rows + i] = acc;
@@ -1232,8 +1298,12 @@ __global__ void k_gnn_reduce(int blocks, int count, const float* __restrict__ pa
 
 // Layer backward, part 1 (tensor cores): dy = dh (.) [y > 0] (kept in BF16
 // for the weight gradient), dcat = dy Wl (128 x 128 per tile, K = 64), then
-// dh += dcat[:, :64] in place and dm = dcat[:, 64:].
-constexpr int kBwdSmem = 1024 + kTile * 128 + 2 * kH * 128;
+// dh += dcat[:, :64] in place and dm = dcat[:, 64:].  A lane holds a TMEM row,
+// so each warp turns its 32 x 32 blocks through shared memory and the rows
+// leave 128 bytes at a time (every lane writing its own row took 103 us for
+// 100,000 vertices, so 29).
+constexpr int kTurn = 36;   // floats per row of the turned block: 16-byte aligned, spread over the banks
+constexpr int kBwdSmem = 1024 + kTile * 128 + 2 * kH * 128 + kTile * kTurn * 4;
 
 __global__ void __launch_bounds__(kLayerThreads, 4)
     k_gnn_layer_bwd(int n, float* __restrict__ dh, const unsigned long long* __restrict__ mask,
@@ -1296,17 +1366,30 @@ __global__ void __launch_bounds__(kLayerThreads, 4)
         ok = wait_phase(bar, iter & 1);
         tmem_fence_after_sync();
         if (!__syncthreads_and(ok)) break;
-        const int v = row0 + 32 * warp + lane;
+        float* turn = reinterpret_cast<float*>(tile + kTile * 128 + 2 * kH * 128) + warp * 32 * kTurn;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             float y[32];
             tmem_ld32(tmem + (static_cast<std::uint32_t>(32 * warp) << 16) + 32 * q, y);
-            if (v < n) {
-                float* dst = q < 2 ? dh + static_cast<long long>(v) * kH + 32 * q
-                                   : dm + static_cast<long long>(v) * kH + 32 * (q - 2);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) dst[i] = q < 2 ? dst[i] + y[i] : y[i];
+            for (int i = 0; i < 32; i += 4)
+                *reinterpret_cast<float4*>(turn + lane * kTurn + i) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
+            __syncwarp();
+            float* out = q < 2 ? dh + 32 * q : dm + 32 * (q - 2);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {   // four rows, eight lanes each
+                const int r = 4 * i + (lane >> 3), v = row0 + 32 * warp + r;
+                float4 x = *reinterpret_cast<const float4*>(turn + r * kTurn + (lane & 7) * 4);
+                if (v < n) {
+                    float4* dst = reinterpret_cast<float4*>(out + static_cast<long long>(v) * kH) + (lane & 7);
+                    if (q < 2) {
+                        const float4 o = *dst;
+                        x = make_float4(o.x + x.x, o.y + x.y, o.z + x.z, o.w + x.w);
+                    }
+                    *dst = x;
+                }
             }
+            __syncwarp();
         }
         tmem_fence_before_sync();
         __syncthreads();
@@ -1337,29 +1420,30 @@ __global__ void __launch_bounds__(256) k_gnn_agg_t(GraphArgs g, const float* __r
 }
 
 // Layer weight gradient on the tensor cores: dWl^T (128 x 64) = [h | m]^T dy,
-// K = vertices.  Each CTA accumulates its tiles in TMEM (operands transposed
-// into K-major shared tiles) and writes one FP32 partial; k_gnn_reduce sums
-// the partials in CTA order.
-constexpr int kWgradSmem = 1024 + 2 * kTile * 128 + 2 * kH * 128;
+// K = vertices.  A tile of 128 vertices is stored as it lies in memory (rows of
+// 64 features, swizzled) and read by the MMA with both operands MN-major, so
+// nothing is transposed; two stages filled by asynchronous copies.  Each CTA
+// accumulates its tiles in TMEM and writes one FP32 partial; k_gnn_reduce sums
+// the partials in CTA order.  Transposing by 2-byte stores into K-major tiles,
+// 71 us for 100,000 vertices; so 13.
+constexpr int kWgradStage = 3 * kTile * 128;   // h, m and dy tiles
+constexpr int kWgradSmem = 1024 + 2 * kWgradStage;
 
-__global__ void __launch_bounds__(kLayerThreads, 4)
+__global__ void __launch_bounds__(kLayerThreads, 2)
     k_gnn_wgrad(int n, const bf16* __restrict__ h, const bf16* __restrict__ m, const bf16* __restrict__ dy,
                 float* __restrict__ partials, unsigned* status)
 {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) std::uint64_t bar_storage;
+    __shared__ __align__(8) std::uint64_t bar_storage[2];
     __shared__ std::uint32_t tmem_base_s;
-    const std::uint32_t raw = smem_u32(smem_raw), base = align1024(raw);
-    unsigned char* tile = smem_raw + (base - raw);
-    // A: 128 feature rows x 128 vertices (two K blocks of 64); B: 64 rows x 128.
-    const std::uint32_t a0 = base, b0 = base + 2 * kTile * 128;
-    const std::uint32_t bar = smem_u32(&bar_storage);
+    const std::uint32_t base = align1024(smem_u32(smem_raw));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ntiles = (n + kTile - 1) / kTile;
     const int t0 = static_cast<int>(static_cast<long long>(ntiles) * blockIdx.x / gridDim.x);
     const int t1 = static_cast<int>(static_cast<long long>(ntiles) * (blockIdx.x + 1) / gridDim.x);
     if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
+        mbar_init(smem_u32(&bar_storage[0]), 1);
+        mbar_init(smem_u32(&bar_storage[1]), 1);
         fence_proxy_async_smem();
     }
     if (warp == 0) tmem_alloc(smem_u32(&tmem_base_s), kH);
@@ -1367,70 +1451,64 @@ __global__ void __launch_bounds__(kLayerThreads, 4)
     __syncthreads();
     tmem_fence_after_sync();
     const std::uint32_t tmem = tmem_base_s;
-    constexpr std::uint32_t idesc = umma_idesc_bf16(kTile, kH);
-    bf16* sa = reinterpret_cast<bf16*>(tile);
-    bf16* sb = reinterpret_cast<bf16*>(tile + 2 * kTile * 128);
-    int iter = 0;
-    bool ok = true;
-    for (int t = t0; t < t1; ++t, ++iter) {
-        const int row0 = t * kTile;
-        // Transpose: vertex k of the tile becomes K index k; feature f a row.
-        for (int i = threadIdx.x; i < kTile * 16; i += kLayerThreads) {
-            const int k = i >> 4, c16 = i & 15, v = row0 + k;     // c16: 16-byte chunk of [h | m] (8 features)
-            uint4 u = make_uint4(0, 0, 0, 0);
-            if (v < n) u = *reinterpret_cast<const uint4*>((c16 < 8 ? h : m) + static_cast<long long>(v) * kH
-                                                          + (c16 & 7) * 8);
-            const bf16* e = reinterpret_cast<const bf16*>(&u);
-            const int kb = k >> 6, kc = (k & 63) >> 3, ke = k & 7;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int f = c16 * 8 + q;
-                sa[(kb * kTile * 128 + sw128(f, kc)) / 2 + ke] = e[q];
-            }
+    constexpr std::uint32_t idesc = umma_idesc_bf16(kTile, kH) | kUmmaMnMajor;
+    // Rows past n are filled with zeros (a copy of no bytes).
+    auto fill = [&](int t, int stage) {
+        const std::uint32_t to = base + stage * kWgradStage;
+        for (int i = threadIdx.x; i < 3 * kTile * 8; i += kLayerThreads) {
+            const int part = i / (kTile * 8), k = i / 8 % kTile, c = i & 7, v = t * kTile + k;
+            const bf16* from = (part == 0 ? h : part == 1 ? m : dy) + static_cast<long long>(min(v, n - 1)) * kH + c * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + part * kTile * 128 + sw128(k, c)),
+                         "l"(from), "r"(v < n ? 16 : 0)
+                         : "memory");
         }
-        for (int i = threadIdx.x; i < kTile * 8; i += kLayerThreads) {
-            const int k = i >> 3, c8 = i & 7, v = row0 + k;
-            uint4 u = make_uint4(0, 0, 0, 0);
-            if (v < n) u = *reinterpret_cast<const uint4*>(dy + static_cast<long long>(v) * kH + c8 * 8);
-            const bf16* e = reinterpret_cast<const bf16*>(&u);
-            const int kb = k >> 6, kc = (k & 63) >> 3, ke = k & 7;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int o = c8 * 8 + q;
-                sb[(kb * kH * 128 + sw128(o, kc)) / 2 + ke] = e[q];
-            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    bool ok = true;
+    if (t0 < t1) fill(t0, 0);
+    for (int t = t0; t < t1 && ok; ++t) {
+        const int iter = t - t0, stage = iter & 1;
+        if (t + 1 < t1) {
+            // The other stage is free once the MMAs of the tile before are done.
+            if (iter > 0) ok = wait_phase(smem_u32(&bar_storage[stage ^ 1]), ((iter - 1) >> 1) & 1);
+            fill(t + 1, stage ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         fence_proxy_async_smem();
         tmem_fence_before_sync();
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        ok = __syncthreads_and(ok);
+        if (threadIdx.x == 0 && ok) {
             tmem_fence_after_sync();
+            const std::uint32_t a0 = base + stage * kWgradStage, b0 = a0 + 2 * kTile * 128;
 #pragma unroll
-            for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    umma_bf16(tmem, umma_desc_sw128(a0 + kb * kTile * 128 + 32 * k),
-                              umma_desc_sw128(b0 + kb * kH * 128 + 32 * k), idesc, iter > 0 || kb > 0 || k > 0);
-            umma_commit(bar);
+            for (int k = 0; k < kTile / 16; ++k)
+                umma_bf16(tmem, umma_desc_sw128_mn(a0 + 2048 * k, kTile * 128), umma_desc_sw128_mn(b0 + 2048 * k, 16),
+                          idesc, iter > 0 || k > 0);
+            umma_commit(smem_u32(&bar_storage[stage]));
         }
-        ok = wait_phase(bar, iter & 1);
-        tmem_fence_after_sync();
-        if (!__syncthreads_and(ok)) break;
     }
+    // The last tile's commit covers every MMA before it.
+    const int last = t1 - t0 - 1;
+    if (last >= 0 && ok) ok = wait_phase(smem_u32(&bar_storage[last & 1]), (last >> 1) & 1);
+    tmem_fence_after_sync();
+    ok = __syncthreads_and(ok);
     // Partial of this CTA (zero if it had no tiles).
     const int f = 32 * warp + lane;
     float* out = partials + static_cast<long long>(blockIdx.x) * (2 * kH) * kH + static_cast<long long>(f) * kH;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         float y[32];
-        if (iter > 0 && ok) {
+        if (last >= 0 && ok) {
             tmem_ld32(tmem + (static_cast<std::uint32_t>(32 * warp) << 16) + 32 * half, y);
         } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) y[i] = 0.0f;
         }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) out[32 * half + i] = y[i];
+        for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(out + 32 * half + i) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
     }
     if (!ok && threadIdx.x == 0) atomicOr(status, kErrTimeout);
     tmem_fence_before_sync();
@@ -1797,18 +1875,14 @@ void gnn_train_buffers(Gnn& G)
 __global__ void k_gnn_features(gnn::GraphArgs g, const double* __restrict__ r, const float* __restrict__ q,
                                const double* norms, float* __restrict__ x)
 {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int v = static_cast<int>(t / gnn::kF), f = static_cast<int>(t % gnn::kF);
     if (v >= g.n) return;
     const double root = sqrt(static_cast<double>(g.n) * g.bs), nr = norms[0], nq = norms[2];
     const float inv_r = nr > 0.0 ? static_cast<float>(root / nr) : 0.0f;
     const float inv_q = nq > 0.0 ? static_cast<float>(root / nq) : 0.0f;
-    float* xv = x + static_cast<long long>(v) * gnn::kF;
-    for (int f = 0; f < gnn::kF; ++f) xv[f] = 0.0f;
-    for (int c = 0; c < g.bs; ++c) {
-        const long long o = static_cast<long long>(v) * g.bs + c;
-        xv[c] = static_cast<float>(r[o]) * inv_r;
-        xv[g.bs + c] = q[o] * inv_q;
-    }
+    const long long o = static_cast<long long>(v) * g.bs;
+    x[t] = f < g.bs ? static_cast<float>(r[o + f]) * inv_r : f < 2 * g.bs ? q[o + f - g.bs] * inv_q : 0.0f;
 }
 
 // Loss and gradient of one (r, e) pair into G.grads; returns the loss.
@@ -1819,7 +1893,7 @@ double gnn_loss_grad(Gnn& G, const double* r, const double* e)
     const gnn::GraphArgs g = G.graph();
     const long long nb = static_cast<long long>(G.n) * G.bs;
     gnn_forward<double, float, true>(G, r, G.out32.as<float>());
-    k_gnn_features<<<G.blocks(G.n), 256, 0, c.stream>>>(g, r, G.qbuf.as<float>(), G.norm_r.as<double>(),
+    k_gnn_features<<<G.blocks(static_cast<long long>(gnn::kF) * G.n), 256, 0, c.stream>>>(g, r, G.qbuf.as<float>(), G.norm_r.as<double>(),
                                                         G.x.as<float>());
     kern::norm<double>(c, static_cast<std::size_t>(nb), e, G.norm_e.as<double>(), G.norm_e.as<double>() + 1);
     gnn::k_gnn_matvec<false><<<G.blocks(nb), 256, 0, c.stream>>>(g, G.nb_a.as<float>(), G.diag_f.as<float>(),
@@ -1835,25 +1909,25 @@ double gnn_loss_grad(Gnn& G, const double* r, const double* e)
                                                    G.loss_partials.as<double>(), G.ticket.as<unsigned>(),
                                                    G.loss.as<double>());
     c.launched(4);
-    gnn::k_gnn_decode_bwd<<<G.blocks(G.n), 256, 0, c.stream>>>(G.n, G.bs, G.dz.as<float>(),
+    gnn::k_gnn_decode_bwd<<<G.blocks(16ll * G.n), 256, 0, c.stream>>>(G.n, G.bs, G.dz.as<float>(),
                                                                 G.params.as<float>() + Gnn::kOffWd, G.dh.as<float>());
     float* grads = G.grads.as<float>();
     OWTK_CUDA(cudaMemsetAsync(grads, 0, Gnn::kParams * sizeof(float), c.stream));
     const unsigned ob = 256;
     gnn::k_gnn_outer<gnn::bf16><<<ob, 256, 0, c.stream>>>(G.n, G.bs, gnn::kH, G.dz.as<float>(),
                                                            G.h[gnn::kLayers].as<gnn::bf16>(), G.partials.as<float>());
-    gnn::k_gnn_reduce<<<G.blocks(G.bs * gnn::kH), 256, 0, c.stream>>>(ob, G.bs * gnn::kH, G.partials.as<float>(),
+    gnn::k_gnn_reduce<<<G.blocks(G.bs * gnn::kH, 32), gnn::kReduceWarps * 32, 0, c.stream>>>(ob, G.bs * gnn::kH, G.partials.as<float>(),
                                                                        grads + Gnn::kOffWd, 0, 0, 0);
     c.launched(6);
     for (int l = gnn::kLayers - 1; l >= 0; --l) {
         gnn::k_gnn_layer_bwd<<<G.layer_grid(), gnn::kLayerThreads, gnn::kBwdSmem, c.stream>>>(
             G.n, G.dh.as<float>(), G.mask[l].as<unsigned long long>(), G.wlt16.as<gnn::bf16>() + l * Gnn::kLayerW,
             G.dy.as<gnn::bf16>(), G.dm.as<float>(), c.status.as<unsigned>());
-        const unsigned wg = G.layer_grid();
+        const unsigned wg = G.layer_grid(2);
         gnn::k_gnn_wgrad<<<wg, gnn::kLayerThreads, gnn::kWgradSmem, c.stream>>>(
             G.n, G.h[l].as<gnn::bf16>(), G.m[l].as<gnn::bf16>(), G.dy.as<gnn::bf16>(), G.partials.as<float>(),
             c.status.as<unsigned>());
-        gnn::k_gnn_reduce<<<G.blocks(2 * gnn::kH * gnn::kH), 256, 0, c.stream>>>(
+        gnn::k_gnn_reduce<<<G.blocks(2 * gnn::kH * gnn::kH, 32), gnn::kReduceWarps * 32, 0, c.stream>>>(
             wg, 2 * gnn::kH * gnn::kH, G.partials.as<float>(), grads + Gnn::kOffWl + l * Gnn::kLayerW, 2 * gnn::kH,
             gnn::kH, 1);
         gnn::k_gnn_agg_t<<<G.blocks(static_cast<long long>(G.n) * 16), 256, 0, c.stream>>>(g, G.dm.as<float>(),
@@ -1863,7 +1937,7 @@ double gnn_loss_grad(Gnn& G, const double* r, const double* e)
     }
     gnn::k_gnn_outer<float><<<ob, 256, 0, c.stream>>>(G.n, gnn::kH, gnn::kF, G.dh.as<float>(), G.x.as<float>(),
                                                        G.partials.as<float>());
-    gnn::k_gnn_reduce<<<G.blocks(gnn::kH * gnn::kF), 256, 0, c.stream>>>(ob, gnn::kH * gnn::kF, G.partials.as<float>(),
+    gnn::k_gnn_reduce<<<G.blocks(gnn::kH * gnn::kF, 32), gnn::kReduceWarps * 32, 0, c.stream>>>(ob, gnn::kH * gnn::kF, G.partials.as<float>(),
                                                                           grads + Gnn::kOffWe, 0, 0, 0);
     OWTK_CUDA(cudaGetLastError());
     c.launched(3);

@@ -39,6 +39,22 @@ __device__ __forceinline__ std::uint64_t umma_desc_sw128(std::uint32_t smem_addr
     return d;
 }
 
+// The same tile read MN-major: the tile's rows are K (8 per swizzle atom, one
+// atom every 1024 bytes), its 64 columns M or N, further blocks of 64 columns
+// `block_bytes` apart.  One MMA consumes two atoms of K, so stepping K by 16
+// adds 2048 bytes to the start address.
+__device__ __forceinline__ std::uint64_t umma_desc_sw128_mn(std::uint32_t smem_addr, std::uint32_t block_bytes)
+{
+    std::uint64_t d = 0;
+    d |= static_cast<std::uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+    d |= static_cast<std::uint64_t>(block_bytes >> 4) << 16;        // leading byte offset: next 64 columns
+    d |= static_cast<std::uint64_t>(1024 >> 4) << 32;               // stride byte offset: next 8 of K
+    d |= static_cast<std::uint64_t>(1) << 46;
+    d |= static_cast<std::uint64_t>(2) << 61;
+    return d;
+}
+constexpr std::uint32_t kUmmaMnMajor = (1u << 15) | (1u << 16);   // instruction descriptor: A and B MN-major
+
 // f16-kind instruction descriptor: BF16 A and B (both K-major), FP32 D.
 __host__ __device__ constexpr std::uint32_t umma_idesc_bf16(int m, int n)
 {

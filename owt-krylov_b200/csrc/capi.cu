@@ -362,11 +362,16 @@ void store_factors(Preconditioner& p)
     if (p.storage == OWTK_F32) {
         kern::convert<float, double>(c, nv, p.d_fvalues.as<double>(), p.lp_vals.as<float>());
         kern::convert<float, double>(c, ni, p.inv_diag.as<double>(), p.lp_inv.as<float>());
-        if (p.upper_local.ready) kern::local_ilu_pack<float, float>(c, p, p.lp_vals.as<float>(), p.lp_inv.as<float>());
+        if (p.upper_local.ready && p.block)
+            kern::local_block_pack<float>(c, p, p.lp_vals.as<float>(), p.lp_inv.as<float>());
+        else if (p.upper_local.ready)
+            kern::local_ilu_pack<float, float>(c, p, p.lp_vals.as<float>(), p.lp_inv.as<float>());
     } else {
         kern::convert<__nv_bfloat16, double>(c, nv, p.d_fvalues.as<double>(), p.lp_vals.as<__nv_bfloat16>());
         kern::convert<__nv_bfloat16, double>(c, ni, p.inv_diag.as<double>(), p.lp_inv.as<__nv_bfloat16>());
-        if (p.upper_local.ready)
+        if (p.upper_local.ready && p.block)
+            kern::local_block_pack<__nv_bfloat16>(c, p, p.lp_vals.as<__nv_bfloat16>(), p.lp_inv.as<__nv_bfloat16>());
+        else if (p.upper_local.ready)
             kern::local_ilu_pack<float, __nv_bfloat16>(c, p, p.lp_vals.as<__nv_bfloat16>(),
                                                        p.lp_inv.as<__nv_bfloat16>());
     }
@@ -1068,6 +1073,7 @@ std::unique_ptr<owtk_preconditioner> make_pc(owtk_matrix* m, owtk_pc_kind kind, 
         if (m->bs > 4) fail(OWTK_ERR_INVALID_ARGUMENT, "block ILU supports block sizes up to 4");
         p->block = true;
         ilu_symbolic(*p, *m, 0);
+        build_local_block_sweep(*p->ctx, *p, storage);
         break;
     }
     default: fail(OWTK_ERR_INVALID_ARGUMENT, "unknown preconditioner kind");

@@ -64,6 +64,15 @@ constexpr int kSharedBytes = 226 * 1024;
 // four warps, as registers allow (at 1,000,000 rows 4, 5 and 6 teams of four
 // took 4,150, 3,730 and 3,260 us).
 constexpr int kTeams1 = 12, kTeams2 = 12, kTeams4 = 6;
+// Dense blocks: teams of one warp, as many as there are named barriers and as
+// their stages leave a ring for.  A visit is some 500 instructions, so what a
+// step costs is the visit over the number of teams (four warps a team, fewer
+// teams: the same at 82 rows a level, two to three times slower below 32).
+constexpr int block_teams(std::size_t stage)
+{
+    return static_cast<int>(std::min<std::size_t>(15, 170 * 1024 / (kDepth * stage)));
+}
+
 // A task's packed word: rows, width << 8, and
 constexpr int kFarFlag = 1 << 24;     // some dependencies are staged from global memory
 constexpr int kSlowFlag = 1 << 25;    // the slower form
@@ -340,9 +349,273 @@ __global__ void __launch_bounds__(W * TEAMS * 32, 1) k_local_sweep(const __grid_
     }
 }
 
+// ---------------------------------------------------------------- dense blocks
+// The same for the dense-block ILU, whose components meet in every row: one
+// CTA for all of them, a lane per row with its BS sums.  (A lane per block row,
+// 32 / BS rows a task, took 1.86 ms where this takes 1.27: as many shared loads
+// for a third of the rows.)  A task's blocks lie
+// [dependency][element][row] in the factor's storage type, BF16 two elements
+// to a word, so a lane's loads neither conflict nor split; a dependency's BS
+// values lie side by side in the ring, padded to 2 or 4.
+// 100,000 rows, bs 3, 82 rows a level, one apply: BF16 factors 2.94 -> 1.27 ms,
+// FP32 2.94 -> 1.09, FP64 3.80 -> 3.04; 4,096 rows, BF16 0.50 -> 0.09.  Bound by
+// the instructions of a visit (46% of the issue slots, shared-memory wavefronts
+// 39%).
+// Padded entries of a task, by the bytes of a block.
+constexpr int block_entries(std::size_t bytes) { return bytes <= 40 ? 128 : 64; }
+
+// Stored elements of a block (BF16: made even).
+template<class F> constexpr int block_elements(int bs) { return sizeof(F) == 2 ? (bs * bs + 1) / 2 * 2 : bs * bs; }
+
+template<class T, class F, int BS>
+struct __align__(16) BlockStage {
+    static constexpr int kEntries = block_entries(sizeof(F) * BS * BS);
+    alignas(16) F coef[kEntries * block_elements<F>(BS)];
+    alignas(16) std::uint16_t slots[kEntries];   // [dependency][row]
+    alignas(16) T own[32 * BS];                       // [row][block row]
+    alignas(16) F dinv[32 * block_elements<F>(BS)];   // [element][row]
+    alignas(16) T far[32 * (BS == 3 ? 4 : BS)];
+    alignas(16) int to[32];
+    alignas(16) int4 task;
+};
+
+template<class T, class F>
+struct BlockArgs {
+    const int4* task;
+    const std::uint16_t* slots;
+    const int* far;
+    const int* to;
+    const F* coef;
+    const F* dinv;           // backward, per task
+    const T* in;             // per place
+    T* out;                  // forward: per place of the backward order; backward: per row
+    int steps, ring;
+};
+
+__device__ __forceinline__ void copy_run(std::uint32_t to, const void* from, int bytes, int lane)
+{
+    for (int o = lane * 16; o < bytes; o += 512) copy16(to + o, static_cast<const char*>(from) + o);
+}
+
+template<class T, class F, int BS, bool BACK>
+__device__ __forceinline__ void load_block(const BlockArgs<T, F>& d, int lane, int4 task, int far,
+                                           BlockStage<T, F, BS>& h)
+{
+    constexpr int kP = BS == 3 ? 4 : BS;
+    const int rows = task.z & 0xff, entries = (rows * (task.z >> 8 & 0xff) + 7) & ~7;
+    constexpr int kE = block_elements<F>(BS);
+    if (lane == 0) h.task = task;
+    if (rows > 0) {
+        const int padded = (rows + 7) & ~7;   // places of a task are padded to 8, entries too
+        copy_run(smem_u32(h.coef), d.coef + static_cast<std::size_t>(task.x) * kE,
+                 entries * kE * static_cast<int>(sizeof(F)), lane);
+        copy_run(smem_u32(h.slots), d.slots + task.x, entries * 2, lane);
+        copy_run(smem_u32(h.own), d.in + static_cast<std::size_t>(task.y) * BS,
+                 padded * BS * static_cast<int>(sizeof(T)), lane);
+        if (BACK)
+            copy_run(smem_u32(h.dinv), d.dinv + static_cast<std::size_t>(task.y) * kE,
+                     padded * kE * static_cast<int>(sizeof(F)), lane);
+        copy_run(smem_u32(h.to), d.to + task.y, padded * 4, lane);
+        if (task.z & kFarFlag && far >= 0) {
+#pragma unroll
+            for (int j = 0; j < BS; ++j)
+                copy_value(smem_u32(h.far) + (lane * kP + j) * static_cast<int>(sizeof(T)),
+                           d.out + static_cast<std::size_t>(far) * BS + j);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template<int BS> __device__ __forceinline__ void ld_block(std::uint32_t a, float (&x)[BS])
+{
+    if constexpr (BS == 1) {
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x[0]) : "r"(a) : "memory");
+    } else if constexpr (BS == 2) {
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x[0]), "=f"(x[1]) : "r"(a) : "memory");
+    } else {
+        float y;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(y) : "r"(a) : "memory");
+        if constexpr (BS == 4) x[3] = y;
+    }
+}
+template<int BS> __device__ __forceinline__ void ld_block(std::uint32_t a, double (&x)[BS])
+{
+    if constexpr (BS == 1) {
+        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x[0]) : "r"(a) : "memory");
+    } else {
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "r"(a) : "memory");
+        if constexpr (BS == 3) {
+            asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x[2]) : "r"(a + 16) : "memory");
+        } else if constexpr (BS == 4) {
+            asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x[2]), "=d"(x[3]) : "r"(a + 16) : "memory");
+        }
+    }
+}
+
 template<class T> __device__ __forceinline__ T widen(double v) { return static_cast<T>(v); }
 template<class T> __device__ __forceinline__ T widen(float v) { return static_cast<T>(v); }
 template<class T> __device__ __forceinline__ T widen(__nv_bfloat16 v) { return static_cast<T>(__bfloat162float(v)); }
+
+// Elements of a block of `at` (row l of a task of `rows`), widened.
+template<class T, class F, int BS>
+__device__ __forceinline__ void load_elements(const F* at, int rows, int l, T (&m)[BS * BS])
+{
+    if constexpr (sizeof(F) == 2) {
+#pragma unroll
+        for (int e = 0; e < block_elements<F>(BS); e += 2) {
+            const unsigned pair = *reinterpret_cast<const unsigned*>(at + e * rows + 2 * l);
+            m[e] = __uint_as_float(pair << 16);
+            if (e + 1 < BS * BS) m[e + 1] = __uint_as_float(pair & 0xffff0000u);
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < BS * BS; ++e) m[e] = at[e * rows + l];
+    }
+}
+
+template<class T, class F, int BS, int N, int PAIR, bool BACK>
+__device__ __forceinline__ void run_block_task(const BlockStage<T, F, BS>& h, const int4& task, int lane,
+                                               std::uint32_t ring, std::uint32_t slot, bool wait, bool signal,
+                                               int wait_id, int signal_id, T (&y)[BS])
+{
+    constexpr int kP = BS == 3 ? 4 : BS, kBytes = kP * static_cast<int>(sizeof(T)), kE = block_elements<F>(BS);
+    const int rows = task.z & 0xff, l = min(lane, rows - 1);
+    std::uint32_t at[N > 0 ? N : 1];
+    T coef[N > 0 ? N : 1][BS * BS], acc[BS], dinv[BS * BS];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const unsigned a = h.slots[k * rows + l];
+        at[k] = ring + a * kBytes;
+        if (task.z & kFarFlag && a >= kFarSlot) at[k] = smem_u32(h.far) + (a - kFarSlot) * kBytes;
+        load_elements<T, F, BS>(h.coef + k * kE * rows, rows, l, coef[k]);
+    }
+#pragma unroll
+    for (int i = 0; i < BS; ++i) acc[i] = h.own[l * BS + i];
+    if (BACK) load_elements<T, F, BS>(h.dinv, rows, l, dinv);
+    if (wait) bar_wait<PAIR>(wait_id);
+    T x[N > 0 ? N : 1][BS];
+#pragma unroll
+    for (int k = 0; k < N; ++k) ld_block<BS>(at[k], x[k]);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+#pragma unroll
+        for (int i = 0; i < BS; ++i) {
+            T sum = T(0);
+#pragma unroll
+            for (int j = 0; j < BS; ++j) sum = add_rn(sum, mul_rn(coef[k][i * BS + j], x[k][j]));
+            acc[i] = sub_rn(acc[i], sum);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < BS; ++i) {
+        if (BACK) {
+            T z = T(0);
+#pragma unroll
+            for (int j = 0; j < BS; ++j) z = add_rn(z, mul_rn(dinv[i * BS + j], acc[j]));
+            y[i] = z;
+        } else {
+            y[i] = acc[i];
+        }
+    }
+    if (lane < rows) {
+#pragma unroll
+        for (int i = 0; i < BS; ++i) st_ring(slot + i * static_cast<int>(sizeof(T)), y[i]);
+    }
+    if (signal) bar_signal<PAIR>(signal_id);
+}
+
+template<class T, class F, int BS, int W, int TEAMS, bool BACK>
+__global__ void __launch_bounds__(W * TEAMS * 32, 1) k_local_block(const __grid_constant__ BlockArgs<T, F> d)
+{
+    constexpr int kP = BS == 3 ? 4 : BS, kSize = static_cast<int>(sizeof(T)), kPair = 2 * W * 32;
+    using Stages = BlockStage<T, F, BS>;
+    extern __shared__ __align__(16) unsigned char shared[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x / 32 % W, team = threadIdx.x / (32 * W);
+    Stages* const stages = reinterpret_cast<Stages*>(shared) + threadIdx.x / 32 * kDepth;
+    const std::uint32_t ring = smem_u32(shared) + W * TEAMS * kDepth * static_cast<int>(sizeof(Stages));
+    if (threadIdx.x < kP) st_ring(ring + (d.ring * kP + threadIdx.x) * kSize, T(0));
+    __syncthreads();
+    const int4* tasks = d.task + w;
+    const int* fars = d.far ? d.far + w * 32 + lane : nullptr;
+    auto task_of = [&](int s) { return s < d.steps ? __ldg(tasks + s * W) : make_int4(0, 0, 0, 0); };
+    auto far_of = [&](int s) { return fars && s < d.steps ? __ldg(fars + static_cast<std::size_t>(s) * W * 32) : -1; };
+    for (int u = 0; u < kDepth; ++u)
+        load_block<T, F, BS, BACK>(d, lane, task_of(team + u * TEAMS), far_of(team + u * TEAMS), stages[u]);
+    int4 next = task_of(team + kDepth * TEAMS);
+    int next_far = far_of(team + kDepth * TEAMS);
+    const int wait_id = 1 + (team + TEAMS - 1) % TEAMS, signal_id = 1 + team;
+    int u = 0;
+    for (int s = team; s < d.steps; s += TEAMS) {
+        Stages& h = stages[u];
+        asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+        __syncwarp();
+        const int4 task = h.task;
+        const int rows = task.z & 0xff, place = task.w + lane;
+        const std::uint32_t slot = ring + (place >= d.ring ? place - d.ring : place) * kP * kSize;
+        const bool wait = s > 0, signal = s + 1 < d.steps;
+        T y[BS];
+        if (rows == 0) {
+            if (wait) bar_wait<kPair>(wait_id);
+            if (signal) bar_signal<kPair>(signal_id);
+        } else {
+            auto run = [&](auto n) {
+                run_block_task<T, F, BS, decltype(n)::value, kPair, BACK>(h, task, lane, ring, slot, wait, signal,
+                                                                          wait_id, signal_id, y);
+            };
+            const int width = task.z >> 8 & 0xff;
+            if (width == 4) run(std::integral_constant<int, 4>());
+            else if (width == 6) run(std::integral_constant<int, 6>());
+            else if (width == 2) run(std::integral_constant<int, 2>());
+            else if (width == 0) run(std::integral_constant<int, 0>());
+            else run(std::integral_constant<int, 8>());
+        }
+        if (lane < rows) {
+            T* out = d.out + static_cast<std::size_t>(h.to[lane]) * BS;
+#pragma unroll
+            for (int i = 0; i < BS; ++i) out[i] = y[i] != y[i] ? Bits<T>::quiet_nan() : y[i];
+        }
+        __syncwarp();
+        load_block<T, F, BS, BACK>(d, lane, next, next_far, h);
+        next = task_of(s + (kDepth + 1) * TEAMS);
+        next_far = far_of(s + (kDepth + 1) * TEAMS);
+        u = u + 1 == kDepth ? 0 : u + 1;
+    }
+}
+
+// Factor blocks, or inverse diagonal blocks (DIAG: one per place), into the
+// order and layout of the tasks; a warp per task.
+template<class F, bool DIAG>
+__global__ void __launch_bounds__(kThreads) k_local_block_pack(std::size_t tasks, int bs, const int4* __restrict__ task,
+                                                               const int* __restrict__ src, const F* __restrict__ from,
+                                                               F* __restrict__ to)
+{
+    const std::size_t t = (static_cast<std::size_t>(blockIdx.x) * kThreads + threadIdx.x) / 32;
+    if (t >= tasks) return;
+    const int4 h = task[t];
+    const int rows = h.z & 0xff, width = DIAG ? 1 : h.z >> 8 & 0xff, b2 = bs * bs;
+    const int elements = sizeof(F) == 2 ? (b2 + 1) / 2 * 2 : b2;
+    const std::size_t first = static_cast<std::size_t>(DIAG ? h.y : h.x);
+    F* out = to + first * elements;
+    for (int e = threadIdx.x % 32; e < rows * width; e += 32) {
+        const int source = src[first + e], k = e / rows, l = e - k * rows;
+        if (source < 0) continue;
+        const F* block = from + static_cast<std::size_t>(source) * b2;
+        for (int m = 0; m < b2; ++m)
+            out[sizeof(F) == 2 ? (k * elements + (m & ~1)) * rows + 2 * l + (m & 1) : (k * elements + m) * rows + l] =
+                block[m];
+    }
+}
+
+// The right-hand side into the forward order.
+template<class T>
+__global__ void __launch_bounds__(kThreads) k_local_block_gather(std::size_t count, int bs, const int* __restrict__ rows,
+                                                                 const T* __restrict__ in, T* __restrict__ to)
+{
+    const std::size_t i = static_cast<std::size_t>(blockIdx.x) * kThreads + threadIdx.x;
+    const std::size_t p = i / bs;
+    if (p < count && rows[p] >= 0) to[i] = in[static_cast<std::size_t>(rows[p]) * bs + i % bs];
+}
 
 // Into the sweep's layout (component-major, order of the steps): coefficients
 // and diagonals of both directions, and the right-hand side.  One thread per
@@ -479,11 +752,18 @@ struct Cut {
     std::vector<std::int32_t> count;   // dependencies per row
 };
 
+// What a task holds: rows, padded entries, and the multiple its places are
+// padded to; dense blocks have their slots [dependency][row] and no slower form.
+struct Shape {
+    int warps, rows, entries, pad;
+    bool block;
+};
+
 // Rows by level and row number, cut into tasks and steps.  (Within a level by
 // number of dependencies, for less padding: the same times.)  False for a row
 // of more dependencies than a task's width holds.
 bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32_t* begin, const std::int32_t* end,
-               const std::int32_t* cols, bool backward, int warps)
+               const std::int32_t* cols, bool backward, const Shape& shape)
 {
     const auto n = static_cast<std::int32_t>(owned);
     cut.count.assign(owned, 0);
@@ -497,12 +777,12 @@ bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32
         std::int32_t e = b;
         while (e < n && level[order[e]] == level[order[b]]) ++e;
         while (b < e) {
-            for (int w = 0; w < warps; ++w) {
+            for (int w = 0; w < shape.warps; ++w) {
                 // As many rows as their padded entries leave room for in a stage.
                 std::int32_t rows = 0, width = 0;
-                while (rows < 32 && b + rows < e) {
+                while (rows < shape.rows && b + rows < e) {
                     const std::int32_t wider = std::max(width, (cut.count[order[b + rows]] + 1) / 2 * 2);
-                    if (rows > 0 && (rows + 1) * wider > kTaskEntries) break;
+                    if (rows > 0 && (rows + 1) * wider > shape.entries) break;
                     width = wider;
                     ++rows;
                 }
@@ -512,7 +792,7 @@ bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32
                     cut.place[order[b + l]] = at + l;
                     cut.rows.push_back(order[b + l]);
                 }
-                while (cut.rows.size() % 4 != 0) cut.rows.push_back(-1);
+                while (cut.rows.size() % shape.pad != 0) cut.rows.push_back(-1);
                 at = static_cast<std::int32_t>(cut.rows.size());
                 b += rows;
             }
@@ -522,10 +802,13 @@ bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32
     return true;
 }
 
-bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t bs, std::size_t element_size,
-                     const Sweep& sweep, Cut& cut, const Cut& other, const std::int32_t* begin, const std::int32_t* end, const std::int32_t* cols,
-                     bool backward, bool with_fin, int warps, int shared_rows)
+// vector_size, value_size: bytes of a vector element and of a stored value.
+bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t bs, std::size_t vector_size,
+                     std::size_t value_size, const Sweep& sweep, Cut& cut, const Cut& other, const std::int32_t* begin,
+                     const std::int32_t* end, const std::int32_t* cols, bool backward, bool with_fin,
+                     const Shape& shape, int shared_rows)
 {
+    const int warps = shape.warps;
     const auto n = static_cast<std::int32_t>(owned);
     const std::vector<std::int32_t>& place = cut.place;
     s.warps = warps;
@@ -553,6 +836,7 @@ bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t
             }
         }
         const bool slow = width > kHold || found > 32;
+        if (slow && shape.block) return false;
         w[0] = static_cast<std::int32_t>(first);
         w[2] |= slow ? kSlowFlag : found > 0 ? kFarFlag : 0;
         w[3] = w[1] % s.ring;
@@ -580,7 +864,8 @@ bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t
                 const std::int32_t from = place[cols[e]];
                 const bool near = p - from <= reach;
                 const std::size_t slot = near ? from % s.ring : kFarSlot + found++ % 32;
-                slots[base + (j & ~std::size_t(1)) * rows + 2 * l + j % 2] = static_cast<std::uint16_t>(slot);
+                slots[shape.block ? base + j * rows + l : base + (j & ~std::size_t(1)) * rows + 2 * l + j % 2] =
+                    static_cast<std::uint16_t>(slot);
                 if (any_slow) code[base + j * rows + l] = near ? from % s.ring : -1 - far_index(cols[e]);
                 src[base + j * rows + l] = e;
                 ++j;
@@ -600,10 +885,16 @@ bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t
     s.src = upload(ctx.stream, src);
     s.rows = upload(ctx.stream, cut.rows);
     s.to = upload(ctx.stream, to);
-    s.coef.allocate(bs * s.entries * element_size + 16);
-    OWTK_CUDA(cudaMemsetAsync(s.coef.ptr, 0, bs * s.entries * element_size, ctx.stream));   // padding: zero
-    if (with_fin) s.fin.allocate(bs * s.places * element_size + 16);
-    s.in.allocate(bs * s.places * element_size + 16);
+    // Values of an entry, and of a row's diagonal.
+    const std::size_t per = !shape.block ? bs : value_size == 2 ? (bs * bs + 1) / 2 * 2 : bs * bs;
+    s.coef.allocate(per * s.entries * value_size + 16);
+    OWTK_CUDA(cudaMemsetAsync(s.coef.ptr, 0, per * s.entries * value_size, ctx.stream));   // padding: zero
+    if (with_fin) {
+        s.fin.allocate(per * s.places * value_size + 16);
+        OWTK_CUDA(cudaMemsetAsync(s.fin.ptr, 0, per * s.places * value_size, ctx.stream));
+    }
+    s.in.allocate(bs * s.places * vector_size + 16);
+    OWTK_CUDA(cudaMemsetAsync(s.in.ptr, 0, bs * s.places * vector_size, ctx.stream));
     s.ready = true;
     return true;
 }
@@ -652,18 +943,137 @@ void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t e
     const int shared_rows =
         static_cast<int>((kSharedBytes - static_cast<std::size_t>(warps * teams_of(warps) * kDepth) * stage) / element_size) - 2;
     Cut lower, upper;
-    if (!cut_steps(lower, p.lower, p.owned, lower_begin, lower_end, cols, false, warps)
-        || !cut_steps(upper, p.upper, p.owned, upper_begin, upper_end, cols, true, warps)) return;
-    if (!build_direction(ctx, p.lower_local, p.owned, p.bs, element_size, p.lower, lower, upper, lower_begin, lower_end, cols,
-                         false, ssor, warps, shared_rows)
-        || !build_direction(ctx, p.upper_local, p.owned, p.bs, element_size, p.upper, upper, lower, upper_begin, upper_end,
-                            cols, true, true, warps, shared_rows)) {
+    const Shape shape{warps, 32, kTaskEntries, 4, false};
+    if (!cut_steps(lower, p.lower, p.owned, lower_begin, lower_end, cols, false, shape)
+        || !cut_steps(upper, p.upper, p.owned, upper_begin, upper_end, cols, true, shape)) return;
+    if (!build_direction(ctx, p.lower_local, p.owned, p.bs, element_size, element_size, p.lower, lower, upper,
+                         lower_begin, lower_end, cols, false, ssor, shape, shared_rows)
+        || !build_direction(ctx, p.upper_local, p.owned, p.bs, element_size, element_size, p.upper, upper, lower,
+                            upper_begin, upper_end, cols, true, true, shape, shared_rows)) {
+        p.lower_local = LocalSweep();
+        p.upper_local = LocalSweep();
+    }
+}
+
+namespace {
+
+template<class T, class F, int BS, bool BACK>
+void launch_block_shape(Context& c, const BlockArgs<T, F>& d)
+{
+    constexpr int kTeams = block_teams(sizeof(BlockStage<T, F, BS>));
+    auto* kernel = k_local_block<T, F, BS, 1, kTeams, BACK>;
+    const int bytes = kTeams * kDepth * static_cast<int>(sizeof(BlockStage<T, F, BS>))
+        + (d.ring + 1) * (BS == 3 ? 4 : BS) * static_cast<int>(sizeof(T));
+    OWTK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes));
+    kernel<<<1, kTeams * 32, bytes, c.stream>>>(d);
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+}
+
+template<class T, class F, bool BACK>
+void launch_block(Context& c, Preconditioner& p, T* out)
+{
+    const LocalSweep& s = BACK ? p.upper_local : p.lower_local;
+    BlockArgs<T, F> d{};
+    d.task = s.task.as<int4>();
+    d.slots = s.slots.as<std::uint16_t>();
+    d.far = s.far.ptr ? s.far.as<int>() : nullptr;
+    d.to = BACK ? s.rows.as<int>() : s.to.as<int>();
+    d.coef = s.coef.as<F>();
+    d.dinv = s.fin.as<F>();
+    d.in = s.in.as<T>();
+    d.out = BACK ? out : p.upper_local.in.as<T>();
+    d.steps = s.steps;
+    d.ring = s.ring;
+    switch (p.bs) {
+    case 1: launch_block_shape<T, F, 1, BACK>(c, d); break;
+    case 2: launch_block_shape<T, F, 2, BACK>(c, d); break;
+    case 3: launch_block_shape<T, F, 3, BACK>(c, d); break;
+    default: launch_block_shape<T, F, 4, BACK>(c, d); break;
+    }
+}
+
+template<class F, bool DIAG>
+void pack_blocks(Context& c, const LocalSweep& s, std::size_t bs, const DeviceBuffer& src, const F* from,
+                 const DeviceBuffer& to)
+{
+    const std::size_t tasks = static_cast<std::size_t>(s.steps) * s.warps;
+    k_local_block_pack<F, DIAG><<<static_cast<unsigned>((tasks * 32 + kThreads - 1) / kThreads), kThreads, 0, c.stream>>>(
+        tasks, static_cast<int>(bs), s.task.as<int4>(), src.as<int>(), from, to.as<F>());
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+}
+
+template<class T, class F> std::size_t block_stage_bytes(std::size_t bs)
+{
+    return bs == 1 ? sizeof(BlockStage<T, F, 1>) : bs == 2 ? sizeof(BlockStage<T, F, 2>)
+        : bs == 3 ? sizeof(BlockStage<T, F, 3>) : sizeof(BlockStage<T, F, 4>);
+}
+
+}  // namespace
+
+// The dense-block ILU's schedule where it pays: its tasks at their cost (BF16,
+// FP32 and FP64 factors, by block size; measured at 82 rows a level, a step
+// being one task) against what a level costs through L2 (1.15 us for FP32
+// vectors, 1.5 us for FP64).
+constexpr double kBlockTaskNs[3][4] = {{105, 110, 160, 210}, {105, 110, 140, 310}, {105, 140, 390, 700}};
+void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage)
+{
+    const char* env = std::getenv("OWTK_LOCAL_SWEEP");   // 0: never
+    if (env && std::atoi(env) == 0) return;
+    const std::size_t n = p.owned, bs = p.bs, vector = storage == OWTK_F64 ? 8 : 4,
+                      value = storage == OWTK_F64 ? 8 : storage == OWTK_F32 ? 4 : 2;
+    const std::size_t stage = storage == OWTK_F64 ? block_stage_bytes<double, double>(bs)
+        : storage == OWTK_F32 ? block_stage_bytes<float, float>(bs) : block_stage_bytes<float, __nv_bfloat16>(bs);
+    const Shape shape{1, 32, block_entries(value * bs * bs), 8, true};
+    const std::size_t stages = block_teams(stage) * kDepth * stage, row = (bs == 3 ? 4 : bs) * vector;
+    if (n == 0 || stages + 1024 * row > kSharedBytes) return;
+    const int shared_rows = static_cast<int>((kSharedBytes - stages) / row) - 2;
+    const std::int32_t *rp = p.f_rowptr.data(), *dp = p.f_diagpos.data(), *ci = p.f_cols.data();
+    std::vector<std::int32_t> after(n);   // first upper entry of each row
+    for (std::size_t r = 0; r < n; ++r) after[r] = dp[r] + 1;
+    Cut lower, upper;
+    if (!cut_steps(lower, p.lower, n, rp, dp, ci, false, shape)
+        || !cut_steps(upper, p.upper, n, after.data(), rp + 1, ci, true, shape)) return;
+    const std::size_t tasks = (lower.task.size() + upper.task.size()) / 4;
+    const double task_ns = kBlockTaskNs[storage == OWTK_F64 ? 2 : storage == OWTK_F32 ? 1 : 0][bs - 1];
+    const double level_ns = storage == OWTK_F64 ? 1400.0 : 1100.0;
+    if (static_cast<double>(tasks) * task_ns > level_ns * (p.lower.depth + p.upper.depth)) return;
+    if (!build_direction(ctx, p.lower_local, n, bs, vector, value, p.lower, lower, upper, rp, dp, ci, false, false, shape,
+                         shared_rows)
+        || !build_direction(ctx, p.upper_local, n, bs, vector, value, p.upper, upper, lower, after.data(), rp + 1, ci,
+                            true, true, shape, shared_rows)) {
         p.lower_local = LocalSweep();
         p.upper_local = LocalSweep();
     }
 }
 
 namespace kern {
+
+template<class F> void local_block_pack(Context& c, Preconditioner& p, const F* factors, const F* inverse)
+{
+    pack_blocks<F, false>(c, p.lower_local, p.bs, p.lower_local.src, factors, p.lower_local.coef);
+    pack_blocks<F, false>(c, p.upper_local, p.bs, p.upper_local.src, factors, p.upper_local.coef);
+    pack_blocks<F, true>(c, p.upper_local, p.bs, p.upper_local.rows, inverse, p.upper_local.fin);
+}
+
+template<class T, class F> void local_block_apply(Context& c, Preconditioner& p, const T* in, T* out)
+{
+    const std::size_t count = p.lower_local.places;
+    k_local_block_gather<T><<<static_cast<unsigned>((count * p.bs + kThreads - 1) / kThreads), kThreads, 0, c.stream>>>(
+        count, static_cast<int>(p.bs), p.lower_local.rows.as<int>(), in, p.lower_local.in.as<T>());
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+    launch_block<T, F, false>(c, p, out);
+    launch_block<T, F, true>(c, p, out);
+}
+
+template void local_block_pack<double>(Context&, Preconditioner&, const double*, const double*);
+template void local_block_pack<float>(Context&, Preconditioner&, const float*, const float*);
+template void local_block_pack<__nv_bfloat16>(Context&, Preconditioner&, const __nv_bfloat16*, const __nv_bfloat16*);
+template void local_block_apply<double, double>(Context&, Preconditioner&, const double*, double*);
+template void local_block_apply<float, float>(Context&, Preconditioner&, const float*, float*);
+template void local_block_apply<float, __nv_bfloat16>(Context&, Preconditioner&, const float*, float*);
 
 template<class T, class F>
 void local_ilu_pack(Context& c, Preconditioner& p, const F* factors, const F* inverse)

@@ -1121,6 +1121,10 @@ template<class T> void ssor_apply(Context& c, Preconditioner& p, const T* in, T*
 // vectors / arithmetic: the inner preconditioner of mixed-precision solves.
 template<class F> void ilu_apply_lp(Context& c, Preconditioner& p, const float* in, float* out)
 {
+    if (p.upper_local.ready && p.block) {
+        local_block_apply<float, F>(c, p, in, out);
+        return;
+    }
     if (p.upper_local.ready) {
         local_ilu_apply<float>(c, p, in, out);
         return;
@@ -1163,10 +1167,16 @@ void block_ilu_factorize(Context& c, Preconditioner& p, const double* matrix_val
     a.upd_target = p.d_upd_target.as<int>();
     a.upd_upper = p.d_upd_upper.as<int>();
     launch<double, double, kBlockFactor>(c, p, p.lower, a);
+    if (p.upper_local.ready && p.storage == OWTK_F64)
+        local_block_pack<double>(c, p, p.d_fvalues.as<double>(), p.inv_diag.as<double>());
 }
 
 void block_ilu_apply(Context& c, Preconditioner& p, const double* in, double* out)
 {
+    if (p.upper_local.ready) {
+        local_block_apply<double, double>(c, p, in, out);
+        return;
+    }
     SweepArgs<double> a{};
     a.rowptr = p.d_frowptr.as<int>();
     a.cols = p.d_fcols.as<int>();

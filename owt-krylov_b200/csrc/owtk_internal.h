@@ -354,6 +354,7 @@ int local_sweep_warps(const Context& ctx, const Sweep& lower, const Sweep& upper
 void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t element_size,
                        const std::int32_t* lower_begin, const std::int32_t* lower_end, const std::int32_t* upper_begin,
                        const std::int32_t* upper_end, const std::int32_t* cols, bool ssor);
+void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage);
 void rcm_order(std::size_t owned, const std::int32_t* rowptr, const std::int32_t* cols,
                std::uint64_t* out);
 void hilbert_order(std::size_t n, const double* xy, std::uint64_t* out);
@@ -441,6 +442,8 @@ template<class T> bool chain_ilu_apply(Context& c, Preconditioner& p, const T* i
 template<class T> bool lockstep_ilu_apply(Context& c, Preconditioner& p, const T* in, T* out);
 template<class T, class F> void local_ilu_pack(Context& c, Preconditioner& p, const F* factors, const F* inverse);
 template<class T> void local_ilu_apply(Context& c, Preconditioner& p, const T* in, T* out);
+template<class F> void local_block_pack(Context& c, Preconditioner& p, const F* factors, const F* inverse);
+template<class T, class F> void local_block_apply(Context& c, Preconditioner& p, const T* in, T* out);
 template<class T>
 void local_ssor_apply(Context& c, Preconditioner& p, const T* values, const T* diag, const T* in, T* out);
 // Test hook: a sweep whose only dependency is never published (bounded wait).

@@ -182,3 +182,56 @@ def test_factor_zero_pivot(native, ctx, problems):
     with pytest.raises(native.OwtkError) as err:
         native.Preconditioner(m, native.PC_ILU, 0)
     assert err.value.kind == "zero_pivot"
+
+
+def _dense(problems, nx, ny, bs, seed, order):
+    rng = np.random.default_rng(seed)
+    xy, edges = problems.lattice(nx, ny, 0.2, rng)
+    return problems.dense_block_system(xy, edges, bs, rng, order=order)
+
+
+@pytest.mark.parametrize("nx,ny,bs,order", [(5, 3, 3, "natural"), (40, 41, 3, "natural"), (33, 60, 2, "rcm"),
+                                            (20, 90, 4, "natural"), (64, 31, 1, "natural"), (120, 110, 3, "rcm")])
+def test_block_ilu(native, ctx, restatement, problems, nx, ny, bs, order):
+    s = _dense(problems, nx, ny, bs, nx, order)
+    n = s.owned
+    m = native.Matrix(ctx, "dense", n, 0, bs, s.rowptr, s.cols, s.vals)
+    p = native.Preconditioner(m, native.PC_BLOCK_ILU, 0)
+    want = restatement.block_ilu(n, bs, s.rowptr, s.cols, s.vals).apply(s.rhs)
+    x = native.Vector(ctx, n, 0, bs).upload(s.rhs)
+    p.apply(x, x)
+    assert_bitwise(x.download(), want, "block ILU(0) in place")
+
+
+@pytest.mark.parametrize("storage", ["F32", "BF16"])
+@pytest.mark.parametrize("nx,ny,bs,order", [(41, 40, 3, "natural"), (60, 33, 2, "rcm"), (30, 50, 4, "rcm"),
+                                            (31, 64, 1, "natural"), (150, 140, 3, "rcm")])
+def test_block_stored_equals_level_scheduled(native, ctx, problems, monkeypatch, storage, nx, ny, bs, order):
+    s = _dense(problems, nx, ny, bs, nx + 1, order)
+    n = s.owned
+    m = native.Matrix(ctx, "dense", n, 0, bs, s.rowptr, s.cols, s.vals)
+    local = native.Preconditioner(m, native.PC_BLOCK_ILU, 0, storage=getattr(native, storage))
+    monkeypatch.setenv("OWTK_LOCAL_SWEEP", "0")
+    levels = native.Preconditioner(m, native.PC_BLOCK_ILU, 0, storage=getattr(native, storage))
+    monkeypatch.delenv("OWTK_LOCAL_SWEEP")
+    x = native.Vector(ctx, n, 0, bs, dtype=np.float32).upload(s.rhs.astype(np.float32))
+    y1, y2 = (native.Vector(ctx, n, 0, bs, dtype=np.float32) for _ in range(2))
+    local.apply(x, y1)
+    levels.apply(x, y2)
+    assert_bitwise(y1.download(), y2.download(), storage)
+
+
+def test_block_ilu_dependencies_beyond_the_ring(native, ctx, restatement):
+    # Levels of 40 rows; every 200th row couples to a row near the start, more
+    # than the ring's rows (3,600 of FP64 3 x 3 blocks) back.
+    n, rp, ci, _ = _rows_system(8000, 1, 9, lambda r, g: [r - 40, r - 41] + ([int(g.integers(0, 100))]
+                                                                           if r > 6000 and r % 200 == 0 else []))
+    rng = np.random.default_rng(2)
+    v = rng.uniform(-0.3, 0.3, size=(ci.size, 3, 3))
+    v[ci == np.repeat(np.arange(n), np.diff(rp))] += 6.0 * np.eye(3)
+    m = native.Matrix(ctx, "dense", n, 0, 3, rp, ci, v.reshape(-1))
+    p = native.Preconditioner(m, native.PC_BLOCK_ILU, 0)
+    x = rng.uniform(-1, 1, n * 3)
+    y = native.Vector(ctx, n, 0, 3)
+    p.apply(native.Vector(ctx, n, 0, 3).upload(x), y)
+    assert_bitwise(y.download(), restatement.block_ilu(n, 3, rp, ci, v.reshape(-1)).apply(x), "block ILU(0)")

@@ -12,7 +12,10 @@
 //
 // Execution.  The grid is co-resident (cooperative launch) and walks a fixed
 // cycle of phases separated by a bounded grid barrier:
-//   SP0 EW0 | { EW1 SP1 EW2 EW3 SP2 EW4 SP3 EW5 }*
+//   SP0 EW0 | { EW1 SP1 EW2 [EW3] SP2 EW4 [SP3 EW5] }*
+// The phases in brackets serve early exits, true residuals and the last
+// iteration; a cycle in which no system asked for them skips them and their
+// barriers (the asking system stamps the cycle, Grid::early / Grid::checks).
 // EW phases are element-wise passes over a static partition of all systems'
 // unknowns (block b owns a contiguous range, cut at system boundaries into
 // segments); SP phases are SpMV passes over a static partition of vertices
@@ -21,8 +24,11 @@
 // vertices-per-warp of the system's block size), lanes over (vertex,
 // component) outputs, entries in row order.  A phase that ends in a
 // reduction writes one partial per segment; the segment that arrives last for
-// its system (ticket) combines that system's partials in segment order and
-// advances the system's state machine.  Systems that are not in a phase's
+// its system (ticket) combines that system's partials and advances the system's
+// state machine: its warp loads them 32 at a time and adds the dots in segment
+// order (one thread walking them, each load behind the other, was most of a
+// phase: 24 systems of 1,000 to 40,000 vertices, 10.8 -> 4.6 ms with the
+// skipped phases and the one-counter barrier).  Systems that are not in a phase's
 // branch skip it; finished systems skip everything, and the launch ends when
 // none is left.
 
@@ -46,7 +52,7 @@ using namespace dev;
 constexpr int kBlock = 256;
 constexpr int kWarps = kBlock / 32;
 constexpr int kEwSlot = 8;          // doubles per element-wise partial: norm A (3), norm B (3), dot
-constexpr int kSpSlot = 2;          // doubles per SpMV partial: two dots
+constexpr int kSpSlot = 2;          // doubles per SpMV partial: two dots (a double2)
 constexpr int kVectors = 9;         // workspace slot order of the reference's bicgstab
 constexpr int kMaxBlockSize = 32;
 constexpr int kBarrierSpin = 1 << 24;
@@ -75,8 +81,10 @@ struct State {               // mutable solver state of one system
 };
 static_assert(sizeof(State) % 8 == 0, "State is copied as 8-byte words");
 
-struct Grid {                // grid barrier
-    unsigned count, gen, abort, pad;
+struct Grid {                // grid barrier; latest cycles + 1 that need the bracketed phases
+    unsigned long long count;   // arrivals since the launch began
+    unsigned abort, pad;
+    unsigned long long early, checks;
 };
 
 struct Options {
@@ -117,37 +125,42 @@ __device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
 __device__ __forceinline__ double* vecp(const Args& a, int v) { return a.vec + static_cast<long long>(v) * a.U; }
 
 // ---------------------------------------------------------------- barrier
-__device__ bool grid_sync(const Args& a)
+// One counter that only grows: an arrival is one releasing add, the wait one
+// acquiring load per poll (`round` barriers so far).  With a generation word,
+// a counter reset by the last arrival and full fences around them, a phase
+// with next to no work took 23 us on 148 blocks.
+__device__ bool grid_sync(const Args& a, unsigned long long& round)
 {
-    __shared__ int ok_s;
+    const unsigned long long target = ++round * gridDim.x;
+    bool ok = true;
     __syncthreads();
     if (threadIdx.x == 0) {
-        int ok = 1;
         Grid* g = a.grid;
-        const unsigned gen = ld_acquire(&g->gen);
-        __threadfence();
-        if (atomicAdd(&g->count, 1u) + 1 == gridDim.x) {
-            atomicExch(&g->count, 0u);
-            __threadfence();
-            st_release(&g->gen, gen + 1);
-        } else {
-            int i = 0;
-            for (; i < kBarrierSpin; ++i) {
-                if (ld_acquire(&g->gen) != gen) break;
-                if (ld_acquire(&g->abort)) break;
-                __nanosleep(64);
-            }
+        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&g->count) : "memory");
+        for (int i = 0;; ++i) {
+            unsigned long long now;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&g->count) : "memory");
+            if (now >= target) break;
             if (i == kBarrierSpin) {
                 atomicOr(a.status, kErrTimeout);
                 st_release(&g->abort, 1u);
             }
+            if ((i & 63) == 63 && ld_acquire(&g->abort)) {
+                ok = false;
+                break;
+            }
+            __nanosleep(20);
         }
-        if (ld_acquire(&g->abort)) ok = 0;
-        __threadfence();
-        ok_s = ok;
     }
-    __syncthreads();
-    return ok_s != 0;
+    return __syncthreads_and(ok);
+}
+
+// Arrival at a system's ticket, after this thread's own partial.
+__device__ __forceinline__ unsigned arrive(unsigned* ticket)
+{
+    unsigned old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ticket) : "memory");
+    return old;
 }
 
 // ---------------------------------------------------------------- state machine
@@ -229,25 +242,52 @@ struct Reduced {
     double d0, d1;
 };
 
-__device__ Reduced combine_ew(const Args& a, const Sys& y)
+// acc + v0 + v1 + ... in lane order (live lanes first), the same in every lane.
+__device__ __forceinline__ double add_lanes(double acc, double v, int live)
 {
-    Reduced r{{0.0, 0.0, 0}, {0.0, 0.0, 0}, 0.0, 0.0};
-    for (int k = 0; k < y.ew_nseg; ++k) {
-        const double* p = a.ew_part + static_cast<long long>(y.ew_slot0 + k) * kEwSlot;
-        r.n0 = norm_merge(r.n0, ScaledSum{ld_cg(p + 0), ld_cg(p + 1), ld_cg(p + 2) != 0.0});
-        r.n1 = norm_merge(r.n1, ScaledSum{ld_cg(p + 3), ld_cg(p + 4), ld_cg(p + 5) != 0.0});
-        r.d0 = add_rn(r.d0, ld_cg(p + 6));
+    if (live == 32) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc = add_rn(acc, __shfl_sync(0xffffffffu, v, j));
+    } else {
+        for (int j = 0; j < live; ++j) acc = add_rn(acc, __shfl_sync(0xffffffffu, v, j));
     }
+    return acc;
+}
+
+// Warp-collective.  Norms merge as a tree over the lanes (they decide, but do
+// not enter the iterates), dots in segment order.
+__device__ Reduced combine_ew(const Args& a, const Sys& y, bool both)
+{
+    const int lane = threadIdx.x & 31;
+    Reduced r{{0.0, 0.0, 0}, {0.0, 0.0, 0}, 0.0, 0.0};
+    for (int k0 = 0; k0 < y.ew_nseg; k0 += 32) {
+        double d = 0.0;
+        if (k0 + lane < y.ew_nseg) {
+            const double* p = a.ew_part + static_cast<long long>(y.ew_slot0 + k0 + lane) * kEwSlot;
+            const ScaledSum n0{ld_cg(p + 0), ld_cg(p + 1), ld_cg(p + 2) != 0.0};
+            d = ld_cg(p + 6);
+            r.n0 = norm_merge(r.n0, n0);
+            if (both) r.n1 = norm_merge(r.n1, ScaledSum{ld_cg(p + 3), ld_cg(p + 4), ld_cg(p + 5) != 0.0});
+        }
+        r.d0 = add_lanes(r.d0, d, min(32, y.ew_nseg - k0));
+    }
+    r.n0 = norm_warp(r.n0);
+    if (both) r.n1 = norm_warp(r.n1);
     return r;
 }
 
-__device__ Reduced combine_sp(const Args& a, const Sys& y)
+__device__ Reduced combine_sp(const Args& a, const Sys& y, bool both)
 {
+    const int lane = threadIdx.x & 31;
     Reduced r{{0.0, 0.0, 0}, {0.0, 0.0, 0}, 0.0, 0.0};
-    for (int k = 0; k < y.sp_nseg; ++k) {
-        const double* p = a.sp_part + static_cast<long long>(y.sp_slot0 + k) * kSpSlot;
-        r.d0 = add_rn(r.d0, ld_cg(p + 0));
-        r.d1 = add_rn(r.d1, ld_cg(p + 1));
+    const double2* part = reinterpret_cast<const double2*>(a.sp_part) + y.sp_slot0;
+    double2 next = lane < y.sp_nseg ? __ldcg(part + lane) : make_double2(0.0, 0.0);
+    for (int k0 = 0; k0 < y.sp_nseg; k0 += 32) {
+        const double2 p = next;
+        if (k0 + 32 + lane < y.sp_nseg) next = __ldcg(part + k0 + 32 + lane);
+        const int live = min(32, y.sp_nseg - k0);
+        r.d0 = add_lanes(r.d0, p.x, live);
+        if (both) r.d1 = add_lanes(r.d1, p.y, live);
     }
     return r;
 }
@@ -263,14 +303,12 @@ __device__ State load_state(const State* p)
     return s;
 }
 
-__device__ void finalize(const Args& a, int phase, int sys)
+__device__ void advance(const Args& a, int phase, int sys, const Reduced& r, unsigned long long cycle)
 {
-    const Sys y = a.sys[sys];
     State s = load_state(a.st + sys);
     const auto& o = a.o;
     switch (phase) {
     case kEw0: {   // r = b - A x, shadow = r; norms of b and r, r.r
-        const Reduced r = combine_ew(a, y);
         s.op_apps += 1;
         s.reductions += 2;
         s.bnorm = norm_value(r.n0);
@@ -294,7 +332,6 @@ __device__ void finalize(const Args& a, int phase, int sys)
         break;
     }
     case kSp1: {   // sv = shadow . A psearch
-        const Reduced r = combine_sp(a, y);
         s.pc_apps += 1;
         s.op_apps += 1;
         s.reductions += 1;
@@ -308,14 +345,12 @@ __device__ void finalize(const Args& a, int phase, int sys)
         break;
     }
     case kEw2: {   // ||mid||
-        const Reduced r = combine_ew(a, y);
         s.reductions += 1;
         s.mnorm = norm_value(r.n0);
         if (s.mnorm <= s.thr) s.flags |= kEarly;
         break;
     }
     case kSp2: {   // omid.mid, omid.omid
-        const Reduced r = combine_sp(a, y);
         s.pc_apps += 1;
         s.op_apps += 1;
         s.reductions += 2;
@@ -333,7 +368,6 @@ __device__ void finalize(const Args& a, int phase, int sys)
         break;
     }
     case kEw4: {
-        const Reduced r = combine_ew(a, y);
         if (s.flags & kEarly) {       // early exit: true residual of x + alpha psearch
             s.op_apps += 1;
             s.reductions += 1;
@@ -363,7 +397,6 @@ __device__ void finalize(const Args& a, int phase, int sys)
         break;
     }
     case kEw5: {   // true residual: replacement / check, or after the last iteration
-        const Reduced r = combine_ew(a, y);
         s.op_apps += 1;
         s.reductions += 1;
         const double tn = norm_value(r.n0);
@@ -386,6 +419,20 @@ __device__ void finalize(const Args& a, int phase, int sys)
         break;
     }
     a.st[sys] = s;
+    // Ask for the bracketed phases: EW3 of this cycle; SP3 and EW5 of this cycle
+    // where they are still ahead, of the next one else.
+    if (phase == kEw2 && s.mode == kRun && (s.flags & kEarly)) atomicMax(&a.grid->early, cycle + 1);
+    if (s.mode == kFinal || (s.mode == kRun && (s.flags & kTrue)))
+        atomicMax(&a.grid->checks, cycle + (phase == kEw5 ? 2 : 1));
+}
+
+// Warp-collective: the system's partials combined, its state advanced.
+__device__ __forceinline__ void finalize(const Args& a, int phase, int sys, unsigned long long cycle)
+{
+    const Sys y = a.sys[sys];
+    const Reduced r = phase == kSp1 || phase == kSp2 ? combine_sp(a, y, phase == kSp2) : combine_ew(a, y, phase == kEw0);
+    if ((threadIdx.x & 31) == 0) advance(a, phase, sys, r, cycle);
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------- SpMV phases
@@ -407,7 +454,10 @@ __device__ __forceinline__ bool sp_role(const Args& a, int phase, int mode, int 
     }
 }
 
-__device__ void sp_phase(const Args& a, int phase)
+// One instance per phase, so that the pointers and sums of one are not live in
+// another; inlined, because calls cost 0.9 ms of the 24 systems' 4.6.
+template<int phase>
+__device__ __forceinline__ void sp_phase(const Args& a, unsigned long long cycle = 0)
 {
     const int wg = blockIdx.x * kWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int s_end = a.sp_first[wg + 1];
@@ -421,7 +471,7 @@ __device__ void sp_phase(const Args& a, int phase)
         if (!sp_role(a, phase, mode, flags, y.bs, vin, vout, dots)) continue;
         const double* in = vin < 0 ? a.x : vecp(a, vin);
         double* out = vecp(a, vout);
-        const double* da = dots ? vecp(a, phase == kSp1 ? kShadow : kMid) : nullptr;
+        const double* da = vecp(a, phase == kSp1 ? kShadow : kMid);
         const int bs = y.bs, vpw = y.vpw;
         double d0 = 0.0, d1 = 0.0;
         for (int v = seg.y; v < seg.z; v += vpw) {
@@ -445,28 +495,22 @@ __device__ void sp_phase(const Args& a, int phase)
                 for (; e < ee; ++e) acc = add_rn(acc, mul_rn(__ldg(vv + (e - eb) * bs), ld_cg(in + __ldg(a.xoff + e) + c)));
                 const long long u = y.u0 + static_cast<long long>(vg - y.v0) * bs + c;
                 out[u] = acc;
-                if (dots == 1) d0 = add_rn(d0, mul_rn(ld_cg(da + u), acc));
-                if (dots == 2) {
+                if (phase == kSp1) d0 = add_rn(d0, mul_rn(ld_cg(da + u), acc));
+                if (phase == kSp2 && dots) {
                     d0 = add_rn(d0, mul_rn(acc, ld_cg(da + u)));
                     d1 = add_rn(d1, mul_rn(acc, acc));
                 }
             }
         }
-        if (dots) {
+        if ((phase == kSp1 || phase == kSp2) && dots) {
             d0 = warp_sum(d0);
-            d1 = warp_sum(d1);
+            if (phase == kSp2) d1 = warp_sum(d1);
+            bool last = false;
             if (lane == 0) {
-                double* p = a.sp_part + static_cast<long long>(seg.w) * kSpSlot;
-                p[0] = d0;
-                p[1] = d1;
-                __threadfence();
-                const unsigned old = atomicAdd(a.tickets + 2 * sys + 1, 1u);
-                if ((old + 1) % static_cast<unsigned>(y.sp_nseg) == 0) {
-                    __threadfence();
-                    finalize(a, phase, sys);
-                }
+                reinterpret_cast<double2*>(a.sp_part)[seg.w] = make_double2(d0, d1);
+                last = (arrive(a.tickets + 2 * sys + 1) + 1) % static_cast<unsigned>(y.sp_nseg) == 0;
             }
-            __syncwarp();
+            if (__shfl_sync(0xffffffffu, last, 0)) finalize(a, phase, sys, cycle);
         }
     }
 }
@@ -479,26 +523,18 @@ __device__ __forceinline__ int ew_role(int phase, int mode, int flags)
     case kEw0: return mode == kRun ? 1 : 0;
     case kEw1: return mode == kRun ? 1 : 0;
     case kEw2: return mode == kRun ? 1 : 0;
-    case kEw3: return mode == kRun ? ((flags & kEarly) ? 2 : 1) : 0;
+    case kEw3: return mode == kRun && (flags & kEarly) ? 1 : 0;
     case kEw4: return mode == kRun ? ((flags & kEarly) ? 2 : 1) : 0;
     case kEw5: return ((mode == kRun && (flags & kTrue)) || mode == kFinal) ? 1 : 0;
     default: return 0;
     }
 }
 
-__device__ void ew_phase(const Args& a, int phase)
+template<int phase>
+__device__ __forceinline__ void ew_phase(const Args& a, unsigned long long cycle = 0)
 {
     __shared__ double red[kWarps][kEwSlot];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double* r = vecp(a, kR);
-    double* shadow = vecp(a, kShadow);
-    double* search = vecp(a, kSearch);
-    double* psearch = vecp(a, kPsearch);
-    double* osearch = vecp(a, kOsearch);
-    double* mid = vecp(a, kMid);
-    double* pmid = vecp(a, kPmid);
-    double* omid = vecp(a, kOmid);
-    double* work = vecp(a, kWork);
     const int s_end = a.ew_first[blockIdx.x + 1];
     for (int sg = a.ew_first[blockIdx.x]; sg < s_end; ++sg) {
         const int4 seg = a.ew_seg[sg];
@@ -507,79 +543,80 @@ __device__ void ew_phase(const Args& a, int phase)
         const int mode = ld_cg(&stp->mode), flags = ld_cg(&stp->flags);
         const int role = ew_role(phase, mode, flags);
         if (role == 0) continue;
-        const double alpha = ld_cg(&stp->alpha), omega = ld_cg(&stp->omega), beta = ld_cg(&stp->beta);
         ScaledSum n0{0.0, 0.0, 0}, n1{0.0, 0.0, 0};
         double d0 = 0.0;
-        bool reduce = true;
-        for (long long u = seg.y + threadIdx.x; u < seg.z; u += kBlock) {
-            switch (phase) {
-            case kEw0: {
-                const double bv = __ldg(a.b + u), rv = sub_rn(bv, ld_cg(work + u));
-                r[u] = rv;
-                shadow[u] = rv;
-                norm_push(n0, bv);
-                norm_push(n1, rv);
+        // One element at a time: loading four ahead took 6.7 ms where this takes
+        // 4.6 (four copies of the norm's update, and registers for them).
+        auto each = [&](auto&& f) {
+            for (long long u = seg.y + threadIdx.x; u < seg.z; u += kBlock) f(u);
+        };
+        auto residual = [&](bool norms_of_b) {   // r = b - work; its norm and r.r
+            each([&](long long u) {
+                const double bv = __ldg(a.b + u), rv = sub_rn(bv, ld_cg(vecp(a, kWork) + u));
+                vecp(a, kR)[u] = rv;
+                if (norms_of_b) {
+                    vecp(a, kShadow)[u] = rv;
+                    norm_push(n0, bv);
+                    norm_push(n1, rv);
+                } else {
+                    norm_push(n0, rv);
+                }
                 d0 = add_rn(d0, mul_rn(rv, rv));
-                break;
-            }
-            case kEw1: {
-                const double rv = ld_cg(r + u);
-                double sv;
+            });
+        };
+        if constexpr (phase == kEw0) {
+            residual(true);
+        } else if constexpr (phase == kEw1) {
+            const double omega = ld_cg(&stp->omega), beta = ld_cg(&stp->beta);
+            each([&](long long u) {
+                const double rv = ld_cg(vecp(a, kR) + u);
+                double v = rv;
                 if (flags & kRestart) {
-                    shadow[u] = rv;
-                    osearch[u] = 0.0;
+                    vecp(a, kShadow)[u] = rv;
+                    vecp(a, kOsearch)[u] = 0.0;
                 }
-                if (flags & kFirst) {
-                    sv = rv;
-                } else {
-                    sv = add_rn(rv, mul_rn(beta, sub_rn(ld_cg(search + u), mul_rn(omega, ld_cg(osearch + u)))));
-                }
-                search[u] = sv;
-                psearch[u] = mul_rn(__ldg(a.inv + u), sv);
-                break;
-            }
-            case kEw2: {
-                const double m = add_rn(mul_rn(1.0, ld_cg(r + u)), mul_rn(-alpha, ld_cg(osearch + u)));
-                mid[u] = m;
+                if (!(flags & kFirst))
+                    v = add_rn(rv, mul_rn(beta, sub_rn(ld_cg(vecp(a, kSearch) + u),
+                                                       mul_rn(omega, ld_cg(vecp(a, kOsearch) + u)))));
+                vecp(a, kSearch)[u] = v;
+                vecp(a, kPsearch)[u] = mul_rn(__ldg(a.inv + u), v);
+            });
+        } else if constexpr (phase == kEw2) {
+            const double alpha = ld_cg(&stp->alpha);
+            each([&](long long u) {
+                const double m = add_rn(mul_rn(1.0, ld_cg(vecp(a, kR) + u)),
+                                        mul_rn(-alpha, ld_cg(vecp(a, kOsearch) + u)));
+                vecp(a, kMid)[u] = m;
+                vecp(a, kPmid)[u] = mul_rn(__ldg(a.inv + u), m);   // not used after an early exit
                 norm_push(n0, m);
-                break;
-            }
-            case kEw3:
-                if (role == 2) a.x[u] = add_rn(ld_cg(a.x + u), mul_rn(alpha, ld_cg(psearch + u)));
-                else pmid[u] = mul_rn(__ldg(a.inv + u), ld_cg(mid + u));
-                break;
-            case kEw4:
-                if (role == 2) {
-                    const double rv = sub_rn(__ldg(a.b + u), ld_cg(work + u));
-                    r[u] = rv;
-                    norm_push(n0, rv);
-                    d0 = add_rn(d0, mul_rn(rv, rv));
-                } else {
-                    const double xv = add_rn(add_rn(ld_cg(a.x + u), mul_rn(alpha, ld_cg(psearch + u))),
-                                             mul_rn(omega, ld_cg(pmid + u)));
-                    const double rv = sub_rn(ld_cg(mid + u), mul_rn(omega, ld_cg(omid + u)));
+            });
+        } else if constexpr (phase == kEw3) {
+            const double alpha = ld_cg(&stp->alpha);
+            each([&](long long u) {
+                a.x[u] = add_rn(ld_cg(a.x + u), mul_rn(alpha, ld_cg(vecp(a, kPsearch) + u)));
+            });
+        } else if constexpr (phase == kEw4) {
+            if (role == 2) {
+                residual(false);
+            } else {
+                const double alpha = ld_cg(&stp->alpha), omega = ld_cg(&stp->omega);
+                each([&](long long u) {
+                    const double xv = add_rn(add_rn(ld_cg(a.x + u), mul_rn(alpha, ld_cg(vecp(a, kPsearch) + u))),
+                                             mul_rn(omega, ld_cg(vecp(a, kPmid) + u)));
+                    const double rv = sub_rn(ld_cg(vecp(a, kMid) + u), mul_rn(omega, ld_cg(vecp(a, kOmid) + u)));
                     a.x[u] = xv;
-                    r[u] = rv;
+                    vecp(a, kR)[u] = rv;
                     norm_push(n0, rv);
-                    d0 = add_rn(d0, mul_rn(ld_cg(shadow + u), rv));
-                }
-                break;
-            case kEw5: {
-                const double rv = sub_rn(__ldg(a.b + u), ld_cg(work + u));
-                r[u] = rv;
-                norm_push(n0, rv);
-                d0 = add_rn(d0, mul_rn(rv, rv));
-                break;
+                    d0 = add_rn(d0, mul_rn(ld_cg(vecp(a, kShadow) + u), rv));
+                });
             }
-            default:
-                break;
-            }
+        } else {
+            residual(false);
         }
-        if (phase == kEw1 || phase == kEw3) reduce = false;
-        if (!reduce) continue;
+        if (phase == kEw1 || phase == kEw3) continue;
         // Block reduction in a fixed order, then the system's ticket.
         n0 = norm_warp(n0);
-        n1 = norm_warp(n1);
+        if (phase == kEw0) n1 = norm_warp(n1);
         d0 = warp_sum(d0);
         if (lane == 0) {
             red[warp][0] = n0.scale;
@@ -591,29 +628,31 @@ __device__ void ew_phase(const Args& a, int phase)
             red[warp][6] = d0;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            ScaledSum m0{red[0][0], red[0][1], red[0][2] != 0.0}, m1{red[0][3], red[0][4], red[0][5] != 0.0};
-            double dd = red[0][6];
-            for (int w = 1; w < kWarps; ++w) {
-                m0 = norm_merge(m0, ScaledSum{red[w][0], red[w][1], red[w][2] != 0.0});
-                m1 = norm_merge(m1, ScaledSum{red[w][3], red[w][4], red[w][5] != 0.0});
-                dd = add_rn(dd, red[w][6]);
+        if (warp == 0) {
+            ScaledSum m0{0.0, 0.0, 0}, m1{0.0, 0.0, 0};
+            double dd = 0.0;
+            if (lane < kWarps) {
+                m0 = ScaledSum{red[lane][0], red[lane][1], red[lane][2] != 0.0};
+                m1 = ScaledSum{red[lane][3], red[lane][4], red[lane][5] != 0.0};
+                dd = red[lane][6];
             }
-            double* p = a.ew_part + static_cast<long long>(seg.w) * kEwSlot;
-            p[0] = m0.scale;
-            p[1] = m0.ssq;
-            p[2] = m0.nan;
-            p[3] = m1.scale;
-            p[4] = m1.ssq;
-            p[5] = m1.nan;
-            p[6] = dd;
-            __threadfence();
-            const Sys y = a.sys[sys];
-            const unsigned old = atomicAdd(a.tickets + 2 * sys, 1u);
-            if ((old + 1) % static_cast<unsigned>(y.ew_nseg) == 0) {
-                __threadfence();
-                finalize(a, phase, sys);
+            m0 = norm_warp(m0);
+            if (phase == kEw0) m1 = norm_warp(m1);
+            double sum = __shfl_sync(0xffffffffu, dd, 0);
+            for (int w = 1; w < kWarps; ++w) sum = add_rn(sum, __shfl_sync(0xffffffffu, dd, w));
+            bool last = false;
+            if (lane == 0) {
+                double* p = a.ew_part + static_cast<long long>(seg.w) * kEwSlot;
+                p[0] = m0.scale;
+                p[1] = m0.ssq;
+                p[2] = m0.nan;
+                p[3] = m1.scale;
+                p[4] = m1.ssq;
+                p[5] = m1.nan;
+                p[6] = sum;
+                last = (arrive(a.tickets + 2 * sys) + 1) % static_cast<unsigned>(a.sys[sys].ew_nseg) == 0;
             }
+            if (__shfl_sync(0xffffffffu, last, 0)) finalize(a, phase, sys, cycle);
         }
         __syncthreads();
     }
@@ -624,12 +663,13 @@ __device__ void ew_phase(const Args& a, int phase)
 // The launch is latency-bound, so more resident warps can outweigh the
 // spills; the autotuner times every count.
 template<int MINB>
-__global__ void __launch_bounds__(kBlock, MINB) k_batch_bicgstab(Args a)
+__global__ void __launch_bounds__(kBlock, MINB) k_batch_bicgstab(const __grid_constant__ Args a)
 {
-    sp_phase(a, kSp0);
-    if (!grid_sync(a)) return;
-    ew_phase(a, kEw0);
-    if (!grid_sync(a)) return;
+    unsigned long long round = 0;
+    sp_phase<kSp0>(a);
+    if (!grid_sync(a, round)) return;
+    ew_phase<kEw0>(a);
+    if (!grid_sync(a, round)) return;
     const long long cap = a.o.maxit + 8;
     for (long long cycle = 0;; ++cycle) {
         if (ld_acquire(a.remaining) == 0) break;
@@ -637,28 +677,35 @@ __global__ void __launch_bounds__(kBlock, MINB) k_batch_bicgstab(Args a)
             if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(a.status, kErrTimeout);
             break;
         }
-        ew_phase(a, kEw1);
-        if (!grid_sync(a)) return;
-        sp_phase(a, kSp1);
-        if (!grid_sync(a)) return;
-        ew_phase(a, kEw2);
-        if (!grid_sync(a)) return;
-        ew_phase(a, kEw3);
-        if (!grid_sync(a)) return;
-        sp_phase(a, kSp2);
-        if (!grid_sync(a)) return;
-        ew_phase(a, kEw4);
-        if (!grid_sync(a)) return;
-        sp_phase(a, kSp3);
-        if (!grid_sync(a)) return;
-        ew_phase(a, kEw5);
-        if (!grid_sync(a)) return;
+        const unsigned long long now = static_cast<unsigned long long>(cycle);
+        ew_phase<kEw1>(a);
+        if (!grid_sync(a, round)) return;
+        sp_phase<kSp1>(a, now);
+        if (!grid_sync(a, round)) return;
+        ew_phase<kEw2>(a, now);
+        if (!grid_sync(a, round)) return;
+        // Every block reads the same stamp: it is written before this barrier
+        // and again only behind later ones.
+        if (__ldcg(&a.grid->early) == now + 1) {
+            ew_phase<kEw3>(a);
+            if (!grid_sync(a, round)) return;
+        }
+        sp_phase<kSp2>(a, now);
+        if (!grid_sync(a, round)) return;
+        ew_phase<kEw4>(a, now);
+        if (!grid_sync(a, round)) return;
+        if (__ldcg(&a.grid->checks) == now + 1) {
+            sp_phase<kSp3>(a);
+            if (!grid_sync(a, round)) return;
+            ew_phase<kEw5>(a, now);
+            if (!grid_sync(a, round)) return;
+        }
     }
 }
 
 // One SpMV pass (psearch -> osearch) over the systems of one block size; the
 // autotuner times it per vertices-per-warp candidate.
-__global__ void __launch_bounds__(kBlock) k_batch_spmv_bench(Args a) { sp_phase(a, kSpBench); }
+__global__ void __launch_bounds__(kBlock) k_batch_spmv_bench(const __grid_constant__ Args a) { sp_phase<kSpBench>(a); }
 
 __global__ void k_batch_init(int nsys, State* st, unsigned* tickets, owtk_solver_result* results, Grid* grid,
                              unsigned* remaining)
@@ -673,7 +720,7 @@ __global__ void k_batch_init(int nsys, State* st, unsigned* tickets, owtk_solver
         results[i] = owtk_solver_result{};
     }
     if (i == 0) {
-        *grid = Grid{0u, 0u, 0u, 0u};
+        *grid = Grid{0ull, 0u, 0u, 0ull, 0ull};
         *remaining = static_cast<unsigned>(nsys);
     }
 }

@@ -1262,10 +1262,11 @@ __global__ void __launch_bounds__(256) k_gnn_outer(int n, int pa, int pb, const 
         *reinterpret_cast<float4*>(partials + static_cast<long long>(blockIdx.x) * pa * pb + i * pb + j) = acc;
 }
 
-// Sum `blocks` partial arrays of `count` floats into out[] (optionally
-// transposed: out[j * rows + i] for element i * cols + j): a block takes 32
-// elements, each of its warps a run of the partial arrays in order, and the
-// runs are added in order.
+// Sum `blocks` partial arrays of `count` floats in block order into out[]
+// (optionally transposed: out[j * rows + i] for element i * cols + j): a block
+// takes 32 elements, its warps bring all the partial arrays' values of them
+// into shared memory side by side, one warp adds them in order (a thread that
+// loads as it adds took 34 us for 592 arrays of 8,192).
 constexpr int kReduceWarps = 8;
 
 __global__ void __launch_bounds__(kReduceWarps * 32) k_gnn_reduce(int blocks, int count,
@@ -1273,21 +1274,16 @@ __global__ void __launch_bounds__(kReduceWarps * 32) k_gnn_reduce(int blocks, in
                                                                   float* __restrict__ out, int rows, int cols,
                                                                   int transpose)
 {
-    __shared__ float runs[kReduceWarps][32];
+    extern __shared__ float staged[];   // [partial array][element]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = blockIdx.x * 32 + lane;
-    const int per = (blocks + kReduceWarps - 1) / kReduceWarps;
-    float acc = 0.0f;
-    if (t < count) {
-        const int end = min(blocks, (w + 1) * per);
 #pragma unroll 16
-        for (int b = w * per; b < end; ++b) acc += __ldg(partials + static_cast<long long>(b) * count + t);
-    }
-    runs[w][lane] = acc;
+    for (int b = w; b < blocks; b += kReduceWarps)
+        staged[b * 32 + lane] = t < count ? __ldg(partials + static_cast<long long>(b) * count + t) : 0.0f;
     __syncthreads();
     if (w != 0 || t >= count) return;
-    acc = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kReduceWarps; ++k) acc += runs[k][lane];
+    float acc = 0.0f;
+#pragma unroll 16
+    for (int b = 0; b < blocks; ++b) acc += staged[b * 32 + lane];
     if (transpose) {
         const int i = t / cols, j = t - i * cols;
         out[j * rows + i] = acc;
@@ -1425,7 +1421,7 @@ __global__ void __launch_bounds__(256) k_gnn_agg_t(GraphArgs g, const float* __r
 // nothing is transposed; two stages filled by asynchronous copies.  Each CTA
 // accumulates its tiles in TMEM and writes one FP32 partial; k_gnn_reduce sums
 // the partials in CTA order.  Transposing by 2-byte stores into K-major tiles,
-// 71 us for 100,000 vertices; so 13.
+// 71 us for 100,000 vertices; so 19.
 constexpr int kWgradStage = 3 * kTile * 128;   // h, m and dy tiles
 constexpr int kWgradSmem = 1024 + 2 * kWgradStage;
 
@@ -1709,6 +1705,7 @@ void gnn_set_attrs()
                                    gnn::kBwdSmem));
     OWTK_CUDA(cudaFuncSetAttribute(gnn::k_gnn_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    gnn::kWgradSmem));
+    OWTK_CUDA(cudaFuncSetAttribute(gnn::k_gnn_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     OWTK_CUDA(cudaFuncSetAttribute(gnn::k_gnn_layer_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    gnn::kTmaSmem));
     OWTK_CUDA(cudaFuncSetAttribute(gnn::k_gnn_layer_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1916,18 +1913,18 @@ double gnn_loss_grad(Gnn& G, const double* r, const double* e)
     const unsigned ob = 256;
     gnn::k_gnn_outer<gnn::bf16><<<ob, 256, 0, c.stream>>>(G.n, G.bs, gnn::kH, G.dz.as<float>(),
                                                            G.h[gnn::kLayers].as<gnn::bf16>(), G.partials.as<float>());
-    gnn::k_gnn_reduce<<<G.blocks(G.bs * gnn::kH, 32), gnn::kReduceWarps * 32, 0, c.stream>>>(ob, G.bs * gnn::kH, G.partials.as<float>(),
+    gnn::k_gnn_reduce<<<G.blocks(G.bs * gnn::kH, 32), gnn::kReduceWarps * 32, ob * 128, c.stream>>>(ob, G.bs * gnn::kH, G.partials.as<float>(),
                                                                        grads + Gnn::kOffWd, 0, 0, 0);
     c.launched(6);
     for (int l = gnn::kLayers - 1; l >= 0; --l) {
         gnn::k_gnn_layer_bwd<<<G.layer_grid(), gnn::kLayerThreads, gnn::kBwdSmem, c.stream>>>(
             G.n, G.dh.as<float>(), G.mask[l].as<unsigned long long>(), G.wlt16.as<gnn::bf16>() + l * Gnn::kLayerW,
             G.dy.as<gnn::bf16>(), G.dm.as<float>(), c.status.as<unsigned>());
-        const unsigned wg = G.layer_grid(2);
+        const unsigned wg = G.layer_grid();
         gnn::k_gnn_wgrad<<<wg, gnn::kLayerThreads, gnn::kWgradSmem, c.stream>>>(
             G.n, G.h[l].as<gnn::bf16>(), G.m[l].as<gnn::bf16>(), G.dy.as<gnn::bf16>(), G.partials.as<float>(),
             c.status.as<unsigned>());
-        gnn::k_gnn_reduce<<<G.blocks(2 * gnn::kH * gnn::kH, 32), gnn::kReduceWarps * 32, 0, c.stream>>>(
+        gnn::k_gnn_reduce<<<G.blocks(2 * gnn::kH * gnn::kH, 32), gnn::kReduceWarps * 32, wg * 128, c.stream>>>(
             wg, 2 * gnn::kH * gnn::kH, G.partials.as<float>(), grads + Gnn::kOffWl + l * Gnn::kLayerW, 2 * gnn::kH,
             gnn::kH, 1);
         gnn::k_gnn_agg_t<<<G.blocks(static_cast<long long>(G.n) * 16), 256, 0, c.stream>>>(g, G.dm.as<float>(),
@@ -1937,7 +1934,7 @@ double gnn_loss_grad(Gnn& G, const double* r, const double* e)
     }
     gnn::k_gnn_outer<float><<<ob, 256, 0, c.stream>>>(G.n, gnn::kH, gnn::kF, G.dh.as<float>(), G.x.as<float>(),
                                                        G.partials.as<float>());
-    gnn::k_gnn_reduce<<<G.blocks(gnn::kH * gnn::kF, 32), gnn::kReduceWarps * 32, 0, c.stream>>>(ob, gnn::kH * gnn::kF, G.partials.as<float>(),
+    gnn::k_gnn_reduce<<<G.blocks(gnn::kH * gnn::kF, 32), gnn::kReduceWarps * 32, ob * 128, c.stream>>>(ob, gnn::kH * gnn::kF, G.partials.as<float>(),
                                                                           grads + Gnn::kOffWe, 0, 0, 0);
     OWTK_CUDA(cudaGetLastError());
     c.launched(3);

@@ -438,12 +438,18 @@ __device__ __forceinline__ void block_partials(const double (&acc)[G], int count
 }
 
 // Last CTA: sum each accumulator's partials over CTAs in a fixed order.
+// The CTA barrier orders every thread's partials before thread 0's fence, and
+// thread 0's second fence before the last CTA's reads: one fence pair per CTA
+// instead of one per warp on each side.
 __device__ __forceinline__ bool last_block(unsigned* ticket)
 {
     __shared__ bool is_last;
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
     __syncthreads();
     return is_last;
 }
@@ -451,7 +457,6 @@ __device__ __forceinline__ bool last_block(unsigned* ticket)
 __device__ __forceinline__ void combine(int count, const double* partials, double* out_dev,
                                         double* out_host)
 {
-    __threadfence();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int j = warp; j < count; j += kThreads / 32) {
         double s = 0;
@@ -653,15 +658,108 @@ __global__ void __launch_bounds__(kThreads, kGsBlocks) k_cgs_update_dot(std::siz
     }
 }
 
-// One-pass scaled 2-norm: each thread keeps (scale, sum of squares relative
-// to scale) and rescales when a larger magnitude arrives; pairs combine the
-// same way.  NaN anywhere gives NaN and an infinite entry gives infinity,
-// as the reference's two-pass scaled norm does (reduction.hpp:64-89).
+// One-pass scaled 2-norm.  A partial is (e, q): the largest biased exponent
+// met, and the sum of squares of the values divided by 2^(e - 1023).  Scaling
+// by a power of two is exact, so no value is divided and partials meet by one
+// exponent maximum and plain sums (a running scale of the largest magnitude
+// divides per value and merges in a serial chain of divisions: 13.6 us at
+// 12,288 values against 8.4 us of a dot).  e is at least 1 (zeros and
+// subnormals) and at most 2045, so the inverse scale is a normal number;
+// e = 0x7ff marks an infinity or NaN, with q = NaN for NaN.  NaN anywhere
+// gives NaN and an infinite entry gives infinity, as the reference's two-pass
+// scaled norm does (reduction.hpp:64-89).
+struct PowSum {
+    unsigned e;
+    double q;
+};
+
+// 2^(-2 d), 0 once it would leave the normal range (the term is then below
+// 2^-1022 of the sum it is added to).
+__device__ __forceinline__ double pow_shift(unsigned d)
+{
+    return d > 511u ? 0.0 : __hiloint2double(static_cast<int>((1023u - 2u * d) << 20), 0);
+}
+
+template<int U> __device__ __forceinline__ void pow_push(PowSum& a, const double (&v)[U])
+{
+    unsigned top = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) top = max(top, static_cast<unsigned>(__double2hiint(v[u])) & 0x7fffffffu);
+    unsigned e = max(top >> 20, a.e);
+    if (e >= 0x7ffu) {   // an infinity or NaN, here or before
+        bool nan = a.e == 0x7ffu && isnan(a.q);
+#pragma unroll
+        for (int u = 0; u < U; ++u) nan = nan || isnan(v[u]);
+        a.e = 0x7ffu;
+        a.q = nan ? __longlong_as_double(0x7ff8000000000000LL) : 1.0;
+        return;
+    }
+    e = min(e, 2045u);
+    const double inverse = __hiloint2double(static_cast<int>((2046u - e) << 20), 0);
+    double q = a.q * pow_shift(e - a.e);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const double t = v[u] * inverse;
+        q = fma(t, t, q);
+    }
+    a.e = e;
+    a.q = q;
+}
+
+__device__ __forceinline__ PowSum pow_warp(PowSum a)
+{
+    const unsigned e = __reduce_max_sync(0xffffffffu, a.e);
+    a.q = warp_sum(a.e == e ? a.q : a.q * pow_shift(e - a.e));
+    a.e = e;
+    return a;
+}
+
+// The CTA's partial, written by warp 0 to slots slot and slot + 1.
+__device__ __forceinline__ void norm_partials(PowSum a, double* partials, int slot)
+{
+    __shared__ PowSum red[kThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    a = pow_warp(a);
+    if (lane == 0) red[warp] = a;
+    __syncthreads();
+    if (warp == 0) {
+        a = pow_warp(lane < kThreads / 32 ? red[lane] : PowSum{1u, 0.0});
+        if (lane == 0) {
+            partials[static_cast<std::size_t>(slot) * gridDim.x + blockIdx.x] = a.q;
+            partials[static_cast<std::size_t>(slot + 1) * gridDim.x + blockIdx.x] = a.e;
+        }
+    }
+}
+
+// Last CTA, one warp: the norm from the CTAs' partials, in a fixed order.
+__device__ __forceinline__ void norm_combine(const double* partials, int slot, double* out_dev, double* out_host)
+{
+    const int lane = threadIdx.x & 31;
+    const double* q = partials + static_cast<std::size_t>(slot) * gridDim.x;
+    const double* e = q + gridDim.x;
+    PowSum a{1u, 0.0};
+    for (unsigned b = lane; b < gridDim.x; b += 32) {
+        const PowSum p{static_cast<unsigned>(__ldcg(e + b)), __ldcg(q + b)};
+        const unsigned top = max(a.e, p.e);
+        const double aq = a.e == top ? a.q : a.q * pow_shift(top - a.e);
+        const double pq = p.e == top ? p.q : p.q * pow_shift(top - p.e);
+        a = PowSum{top, aq + pq};
+    }
+    a = pow_warp(a);
+    if (lane == 0) {
+        double r;
+        if (a.e == 0x7ffu) r = isnan(a.q) ? a.q : __longlong_as_double(0x7ff0000000000000LL);
+        else r = __hiloint2double(static_cast<int>(a.e << 20), 0) * sqrt(a.q);
+        *out_dev = r;
+        *out_host = r;
+    }
+}
+
 template<class T>
 __global__ void __launch_bounds__(kThreads) k_norm(std::size_t n, const T* __restrict__ x, double* partials,
                                                    unsigned* ticket, double* out_dev, double* out_host)
 {
-    ScaledSum a{0.0, 0.0, 0};
+    PowSum a{1u, 0.0};
     const std::size_t stride = static_cast<std::size_t>(gridDim.x) * kThreads;
     constexpr int kU = 8;   // loads in flight per thread
     for (std::size_t i = static_cast<std::size_t>(blockIdx.x) * kThreads + threadIdx.x; i < n; i += kU * stride) {
@@ -671,46 +769,101 @@ __global__ void __launch_bounds__(kThreads) k_norm(std::size_t n, const T* __res
             const std::size_t idx = i + u * stride;
             v[u] = idx < n ? static_cast<double>(x[idx]) : 0.0;
         }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) norm_push(a, v[u]);
+        pow_push(a, v);
     }
-    a = norm_warp(a);
-    __shared__ ScaledSum red[kThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) red[warp] = a;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ScaledSum s = red[0];
-        for (int w = 1; w < kThreads / 32; ++w) s = norm_merge(s, red[w]);
-        partials[3 * blockIdx.x + 0] = s.scale;
-        partials[3 * blockIdx.x + 1] = s.ssq;
-        partials[3 * blockIdx.x + 2] = s.nan;
-    }
+    norm_partials(a, partials, 0);
     if (last_block(ticket)) {
-        __threadfence();
-        // Every thread merges a strided share of the CTA partials, then the
-        // CTA merges the threads' results (fixed order: deterministic).
-        ScaledSum t{0.0, 0.0, 0};
-        for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads) {
-            const ScaledSum p{__ldcg(partials + 3 * b), __ldcg(partials + 3 * b + 1),
-                              __ldcg(partials + 3 * b + 2) != 0.0};
-            t = norm_merge(t, p);
+        if (threadIdx.x < 32) norm_combine(partials, 0, out_dev, out_host);
+        if (threadIdx.x == 0) *ticket = 0;
+    }
+}
+
+// BiCGSTAB's two vector updates with the norm that follows each, in one pass
+// and one launch: the updated vector is reduced from registers instead of
+// being read back, and at small sizes, where a launch and the host's wait for
+// a scalar are most of the time, an iteration has two launches fewer.  The
+// norms only meet thresholds; the dots stay in their own kernel, because a
+// differently compiled copy of its loop contracts other products into fused
+// multiply-adds and the iteration amplifies the last bit of rho (the final
+// residual of a 12,288-unknown Jacobi solve then moves in its second to
+// fourth digit).
+
+// mid = r + minus_alpha v; |mid|.
+template<class T>
+__global__ void __launch_bounds__(kThreads) k_bicg_mid(std::size_t n, const T* __restrict__ r, T minus_alpha,
+                                                       const T* __restrict__ v, T* __restrict__ mid,
+                                                       double* partials, unsigned* ticket, double* out_dev,
+                                                       double* out_host)
+{
+    PowSum a{1u, 0.0};
+    const std::size_t stride = static_cast<std::size_t>(gridDim.x) * kThreads;
+    constexpr int kU = 8;
+    for (std::size_t i = static_cast<std::size_t>(blockIdx.x) * kThreads + threadIdx.x; i < n; i += kU * stride) {
+        T rv[kU], vv[kU];
+        double m[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const std::size_t idx = i + u * stride;
+            rv[u] = idx < n ? r[idx] : T(0);
+            vv[u] = idx < n ? v[idx] : T(0);
         }
-        t = norm_warp(t);
-        __syncthreads();
-        if (lane == 0) red[warp] = t;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            ScaledSum s = red[0];
-            for (int w = 1; w < kThreads / 32; ++w) s = norm_merge(s, red[w]);
-            double r;
-            if (s.nan) r = __longlong_as_double(0x7ff8000000000000LL);
-            else if (s.scale == 0.0 || isinf(s.scale)) r = s.scale;
-            else r = s.scale * sqrt(s.ssq);
-            *out_dev = r;
-            *out_host = r;
-            *ticket = 0;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const std::size_t idx = i + u * stride;
+            const T value = add_rn(rv[u], mul_rn(minus_alpha, vv[u]));
+            if (idx < n) mid[idx] = value;
+            m[u] = idx < n ? static_cast<double>(value) : 0.0;
         }
+        pow_push(a, m);
+    }
+    norm_partials(a, partials, 0);
+    if (last_block(ticket)) {
+        if (threadIdx.x < 32) norm_combine(partials, 0, out_dev, out_host);
+        if (threadIdx.x == 0) *ticket = 0;
+    }
+}
+
+// x += alpha ph; x += omega sh; r = s - omega t   (krylov_solvers.hpp:703-708); |r|.
+template<class T>
+__global__ void __launch_bounds__(kThreads, 3)
+    k_bicg_xr_norm(std::size_t n, T alpha, const T* __restrict__ ph, T omega, const T* __restrict__ sh,
+                   const T* __restrict__ s, const T* __restrict__ t, T* __restrict__ x, T* __restrict__ r,
+                   double* partials, unsigned* ticket, double* out_dev, double* out_host)
+{
+    PowSum a{1u, 0.0};
+    const std::size_t stride = static_cast<std::size_t>(gridDim.x) * kThreads;
+    constexpr int kU = 4;
+    for (std::size_t i = static_cast<std::size_t>(blockIdx.x) * kThreads + threadIdx.x; i < n; i += kU * stride) {
+        T xv[kU], pv[kU], hv[kU], sv[kU], tv[kU];
+        double m[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const std::size_t idx = i + u * stride;
+            const bool on = idx < n;
+            xv[u] = on ? x[idx] : T(0);
+            pv[u] = on ? ph[idx] : T(0);
+            hv[u] = on ? sh[idx] : T(0);
+            sv[u] = on ? s[idx] : T(0);
+            tv[u] = on ? t[idx] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const std::size_t idx = i + u * stride;
+            const T rv = sub_rn(sv[u], mul_rn(omega, tv[u]));
+            if (idx < n) {
+                x[idx] = add_rn(add_rn(xv[u], mul_rn(alpha, pv[u])), mul_rn(omega, hv[u]));
+                r[idx] = rv;
+                m[u] = static_cast<double>(rv);
+            } else {
+                m[u] = 0.0;
+            }
+        }
+        pow_push(a, m);
+    }
+    norm_partials(a, partials, 0);
+    if (last_block(ticket)) {
+        if (threadIdx.x < 32) norm_combine(partials, 0, out_dev, out_host);
+        if (threadIdx.x == 0) *ticket = 0;
     }
 }
 
@@ -1318,6 +1471,24 @@ template<class T> void norm(Context& c, std::size_t n, const T* x, double* out_d
     c.launched();
 }
 
+template<class T> void bicg_mid_norm(Context& c, std::size_t n, const T* r, T minus_alpha, const T* v, T* mid,
+                                     double* out_dev, double* out_host)
+{
+    k_bicg_mid<T><<<reduce_blocks(c, n), kThreads, 0, c.stream>>>(n, r, minus_alpha, v, mid, partials_of(c),
+                                                                  ticket_of(c), out_dev, out_host);
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+}
+
+template<class T> void bicg_xr_norm(Context& c, std::size_t n, T alpha, const T* ph, T omega, const T* sh, const T* s,
+                                    const T* t, T* x, T* r, double* out_dev, double* out_host)
+{
+    k_bicg_xr_norm<T><<<reduce_blocks(c, n), kThreads, 0, c.stream>>>(
+        n, alpha, ph, omega, sh, s, t, x, r, partials_of(c), ticket_of(c), out_dev, out_host);
+    OWTK_CUDA(cudaGetLastError());
+    c.launched();
+}
+
 template<class T> void permute_nodes(Context& c, std::size_t n, std::size_t bs, const std::int64_t* n2o, const T* src,
                                      T* dst, bool inverse)
 {
@@ -1429,6 +1600,9 @@ template void convert<__nv_bfloat16, double>(Context&, std::size_t, const double
     template void multidot<T>(Context&, std::size_t, int, const T* const*, const T* const*, double*, double*); \
     template void cgs_update_dot<T>(Context&, std::size_t, int, const T* const*, const double*, T*, double*, double*); \
     template void norm<T>(Context&, std::size_t, const T*, double*, double*);                       \
+    template void bicg_mid_norm<T>(Context&, std::size_t, const T*, T, const T*, T*, double*, double*); \
+    template void bicg_xr_norm<T>(Context&, std::size_t, T, const T*, T, const T*, const T*, const T*, T*, T*, \
+                                  double*, double*);                                                   \
     template void multidot_accurate<T>(Context&, std::size_t, int, int, const T* const*, const T* const*,  \
                                        double*, double*, double*);                                 \
     template void norm_accurate<T>(Context&, std::size_t, const T*, double*, double*, double*);      \

@@ -406,6 +406,12 @@ template<class T> void gmres_update(Context& c, std::size_t n, int k, const T* c
 template<class T> void multidot(Context& c, std::size_t n, int k, const T* const* a,
                                 const T* const* b, double* out_dev, double* out_host);
 template<class T> void norm(Context& c, std::size_t n, const T* x, double* out_dev, double* out_host);
+// BiCGSTAB: mid = r + minus_alpha v with |mid| in out[0].
+template<class T> void bicg_mid_norm(Context& c, std::size_t n, const T* r, T minus_alpha, const T* v, T* mid,
+                                     double* out_dev, double* out_host);
+// bicg_xr with |r| in out[0].
+template<class T> void bicg_xr_norm(Context& c, std::size_t n, T alpha, const T* ph, T omega, const T* sh, const T* s,
+                                    const T* t, T* x, T* r, double* out_dev, double* out_host);
 // Accurate reductions: mode 1 compensated (Neumaier over rounded products),
 // mode 2 doubled precision (TwoProduct + TwoSum, the Dot2 algorithm).  out_lo
 // (host, may be null) receives the low part: out + out_lo is the pair's exact sum.

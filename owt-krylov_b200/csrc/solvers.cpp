@@ -219,6 +219,11 @@ void bicgstab(Engine<T>& e, Vector& b, Vector& x, Workspace& ws)
     if (r0 <= thr) { res.status = kConverged; return; }
 
     T rho_prev = 1, alpha = 1, omega = 1;
+    // With plain sums the vector updates carry the norm that follows them, and
+    // the next rho = shadow . r is enqueued with |r|: one wait for both.
+    const bool fused = e.mode() == 0;
+    T next_rho = 0;
+    bool have_rho = false;
     bool first = true;
     auto restart = [&]() {
         e.copy(r, shadow);
@@ -226,10 +231,17 @@ void bicgstab(Engine<T>& e, Vector& b, Vector& x, Workspace& ws)
         e.fill(osearch, T(0));
         rho_prev = 1; alpha = 1; omega = 1;
         first = true;
+        have_rho = false;
     };
     for (std::uint64_t it = 1; it <= o.maximum_iterations; ++it) {
         res.iterations = it;
-        const T rho = e.dot(shadow, r);
+        T rho;
+        if (have_rho) {
+            rho = next_rho;
+            ++res.global_reductions;
+        } else {
+            rho = e.dot(shadow, r);
+        }
         if (!std::isfinite(rho) || std::abs(rho) <= tiny) {
             e.breakdown(std::isfinite(rho) ? kBiorthogonality : kNonFinite);
             return;
@@ -250,8 +262,16 @@ void bicgstab(Engine<T>& e, Vector& b, Vector& x, Workspace& ws)
             return;
         }
         alpha = rho / sv;
-        kern::lincomb<T>(e.c, e.n, T(1), e.p(r), -alpha, e.p(osearch), e.p(mid));
-        const T mnorm = e.norm(mid);
+        T mnorm;
+        if (fused) {
+            kern::bicg_mid_norm<T>(e.c, e.n, e.p(r), -alpha, e.p(osearch), e.p(mid), e.dslot(kSlotA), e.hslot(kSlotA));
+            ++res.global_reductions;
+            e.c.sync();
+            mnorm = e.scalar(kSlotA);
+        } else {
+            kern::lincomb<T>(e.c, e.n, T(1), e.p(r), -alpha, e.p(osearch), e.p(mid));
+            mnorm = e.norm(mid);
+        }
         if (mnorm <= thr) {
             e.axpy(alpha, psearch, x);
             if (e.app_converged(b, x)) return;
@@ -279,12 +299,27 @@ void bicgstab(Engine<T>& e, Vector& b, Vector& x, Workspace& ws)
             e.breakdown(std::isfinite(omega) ? kOmegaZero : kNonFinite);
             return;
         }
-        kern::bicg_xr<T>(e.c, e.n, alpha, e.p(psearch), omega, e.p(pmid), e.p(mid), e.p(omid), e.p(x), e.p(r));
+        T rnorm = 0;
+        if (fused) {
+            kern::bicg_xr_norm<T>(e.c, e.n, alpha, e.p(psearch), omega, e.p(pmid), e.p(mid), e.p(omid), e.p(x), e.p(r),
+                                  e.dslot(kSlotA), e.hslot(kSlotA));
+            const T* da1[1] = {e.p(shadow)};
+            const T* db1[1] = {e.p(r)};
+            kern::multidot<T>(e.c, e.n, 1, da1, db1, e.dslot(kSlotA + 1), e.hslot(kSlotA + 1));
+            e.c.sync();
+            rnorm = e.scalar(kSlotA);
+            next_rho = e.scalar(kSlotA + 1);
+            have_rho = true;
+        } else {
+            kern::bicg_xr<T>(e.c, e.n, alpha, e.p(psearch), omega, e.p(pmid), e.p(mid), e.p(omid), e.p(x), e.p(r));
+        }
         if (e.app_converged(b, x)) return;
         const bool replace = o.residual_replacement_interval > 0 && it % o.residual_replacement_interval == 0;
         const bool check = !e.has_test() && it % o.convergence_check_interval == 0;
         if (replace || check) {
-            const T rn = e.norm(r);
+            if (fused) ++res.global_reductions;
+            else rnorm = e.norm(r);
+            const T rn = rnorm;
             if (replace || rn <= thr) {
                 e.true_residual(b, x, r, work);
                 const T tn = e.norm(r);

@@ -185,7 +185,8 @@ owtk_status owtk_pc_levels(owtk_preconditioner* pc, int32_t* lower_level, int32_
  * counterpart): cluster_ctas > 0 when they run on one thread-block cluster of
  * that many CTAs (dependency values through distributed shared memory, epochs
  * of epoch_levels levels, ring_rows rows of results per CTA), 0 for the
- * level-scheduled sweep over the whole GPU.  Both give the same bits.  The
+ * default: one CTA per component while the levels are narrow, else the
+ * level-scheduled sweep over the whole GPU.  All give the same bits.  The
  * cluster schedule is opt-in (environment variable OWTK_CLUSTER_SWEEP=1 at
  * preconditioner creation): on a 2M-vertex RCM-ordered mesh it measured
  * slower than the level-scheduled sweep. */

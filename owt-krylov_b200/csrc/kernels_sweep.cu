@@ -1,6 +1,11 @@
 // Level-scheduled triangular sweeps (sm_100a): ILU(k) numeric factorisation,
 // ILU forward/backward solves and SSOR forward/backward sweeps.
 //
+// This is the schedule for wide levels.  While the levels are narrow, ILU and
+// SSOR applies run on one CTA per component instead (kernels_local_sweep.cu),
+// and rows of up to 16 entries are factorised by k_ilu_factor below, which
+// synchronises on the factor's values.
+//
 // Schedule (built once at symbolic setup, reused by every numeric update and
 // apply): rows are ordered by (level, row) and cut into warp tasks of up to
 // 32/bs rows from a single level, so rows inside a task never depend on each
@@ -22,7 +27,7 @@
 // that mesh 150.6 -> 92.3 ms).  A second poll round in flight, half a round
 // trip behind the first, was slower (5.0 -> 9.6 ms): the polls and the spin
 // that staggers them cost more issue and L2 traffic than they save.
-// The numeric factorisation, which updates factor entries in
+// The numeric factorisation of longer rows, which updates factor entries in
 // place, publishes per-row epoch flags instead (fence + release / relaxed
 // loads + fence).  Every wait is bounded (kSpinLimit polls): a wait that gives
 // up sets the timeout bit of the device status word and carries on, and later

@@ -44,6 +44,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <future>
 #include <type_traits>
 
 #include <cuda_bf16.h>
@@ -802,11 +803,18 @@ bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32
     return true;
 }
 
-// vector_size, value_size: bytes of a vector element and of a stored value.
-bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t bs, std::size_t vector_size,
-                     std::size_t value_size, const Sweep& sweep, Cut& cut, const Cut& other, const std::int32_t* begin,
-                     const std::int32_t* end, const std::int32_t* cols, bool backward, bool with_fin,
-                     const Shape& shape, int shared_rows)
+// A direction's tables on the host.
+struct Plan {
+    std::vector<std::int32_t> far, code, src, to;
+    std::vector<std::uint16_t> slots;
+};
+
+// Fills the sizes of s, the tasks of cut and the plan; false where the
+// direction does not suit the schedule.  Touches nothing of the other
+// direction but its places, and no CUDA call.
+bool plan_direction(Plan& plan, LocalSweep& s, std::size_t owned, const Sweep& sweep, Cut& cut, const Cut& other,
+                    const std::int32_t* begin, const std::int32_t* end, const std::int32_t* cols, bool backward,
+                    const Shape& shape, int shared_rows)
 {
     const int warps = shape.warps;
     const auto n = static_cast<std::int32_t>(owned);
@@ -820,7 +828,7 @@ bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t
     auto needed = [&](std::int32_t row, std::int32_t col) { return backward ? col > row && col < n : col < row; };
     auto far_index = [&](std::int32_t col) { return backward ? col : other.place[col]; };
     std::size_t first = 0, used = 0, slow_tasks = 0;
-    std::vector<std::int32_t> far;
+    std::vector<std::int32_t>& far = plan.far;
     for (std::size_t t = 0; t < cut.task.size(); t += 4) {
         std::int32_t* w = cut.task.data() + t;
         const std::int32_t rows = w[2] & 0xff, width = w[2] >> 8;
@@ -851,8 +859,9 @@ bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t
     // a level of the level-scheduled sweep.
     if (slow_tasks > static_cast<std::size_t>(sweep.depth) / 4) return false;
     const bool any_slow = slow_tasks > 0;
-    std::vector<std::int32_t> code(any_slow ? s.entries : 0, s.ring), src(s.entries, -1);
-    std::vector<std::uint16_t> slots(s.entries, static_cast<std::uint16_t>(s.ring));
+    plan.code.assign(any_slow ? s.entries : 0, s.ring);
+    plan.src.assign(s.entries, -1);
+    plan.slots.assign(s.entries, static_cast<std::uint16_t>(s.ring));
     for (std::size_t t = 0; t < cut.task.size(); t += 4) {
         const std::size_t base = static_cast<std::size_t>(cut.task[t]), rows = cut.task[t + 2] & 0xff;
         std::size_t found = 0;
@@ -864,27 +873,34 @@ bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t
                 const std::int32_t from = place[cols[e]];
                 const bool near = p - from <= reach;
                 const std::size_t slot = near ? from % s.ring : kFarSlot + found++ % 32;
-                slots[shape.block ? base + j * rows + l : base + (j & ~std::size_t(1)) * rows + 2 * l + j % 2] =
+                plan.slots[shape.block ? base + j * rows + l : base + (j & ~std::size_t(1)) * rows + 2 * l + j % 2] =
                     static_cast<std::uint16_t>(slot);
-                if (any_slow) code[base + j * rows + l] = near ? from % s.ring : -1 - far_index(cols[e]);
-                src[base + j * rows + l] = e;
+                if (any_slow) plan.code[base + j * rows + l] = near ? from % s.ring : -1 - far_index(cols[e]);
+                plan.src[base + j * rows + l] = e;
                 ++j;
             }
         }
     }
-    std::vector<std::int32_t> to;
     if (!backward) {
-        to.assign(s.places, 0);
+        plan.to.assign(s.places, 0);
         for (std::size_t p = 0; p < s.places; ++p)
-            if (cut.rows[p] >= 0) to[p] = other.place[cut.rows[p]];
+            if (cut.rows[p] >= 0) plan.to[p] = other.place[cut.rows[p]];
     }
+    return true;
+}
+
+// The plan on the device.  vector_size, value_size: bytes of a vector element
+// and of a stored value.
+void place_direction(Context& ctx, LocalSweep& s, const Plan& plan, const Cut& cut, std::size_t bs,
+                     std::size_t vector_size, std::size_t value_size, bool with_fin, const Shape& shape)
+{
     s.task = upload(ctx.stream, cut.task);
-    s.slots = upload(ctx.stream, slots);
-    if (!far.empty()) s.far = upload(ctx.stream, far);
-    if (any_slow) s.code = upload(ctx.stream, code);
-    s.src = upload(ctx.stream, src);
+    s.slots = upload(ctx.stream, plan.slots);
+    if (!plan.far.empty()) s.far = upload(ctx.stream, plan.far);
+    if (!plan.code.empty()) s.code = upload(ctx.stream, plan.code);
+    s.src = upload(ctx.stream, plan.src);
     s.rows = upload(ctx.stream, cut.rows);
-    s.to = upload(ctx.stream, to);
+    s.to = upload(ctx.stream, plan.to);
     // Values of an entry, and of a row's diagonal.
     const std::size_t per = !shape.block ? bs : value_size == 2 ? (bs * bs + 1) / 2 * 2 : bs * bs;
     s.coef.allocate(per * s.entries * value_size + 16);
@@ -896,7 +912,15 @@ bool build_direction(Context& ctx, LocalSweep& s, std::size_t owned, std::size_t
     s.in.allocate(bs * s.places * vector_size + 16);
     OWTK_CUDA(cudaMemsetAsync(s.in.ptr, 0, bs * s.places * vector_size, ctx.stream));
     s.ready = true;
-    return true;
+}
+
+// Both directions side by side, the lower one on another thread where one can
+// be had.
+template<class L, class U> bool both(L lower, U upper)
+{
+    std::future<bool> first = std::async(lower);
+    const bool second = upper();
+    return first.get() && second;
 }
 
 constexpr int teams_of(int warps) { return warps == 1 ? kTeams1 : warps == 2 ? kTeams2 : kTeams4; }
@@ -944,15 +968,19 @@ void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t e
         static_cast<int>((kSharedBytes - static_cast<std::size_t>(warps * teams_of(warps) * kDepth) * stage) / element_size) - 2;
     Cut lower, upper;
     const Shape shape{warps, 32, kTaskEntries, 4, false};
-    if (!cut_steps(lower, p.lower, p.owned, lower_begin, lower_end, cols, false, shape)
-        || !cut_steps(upper, p.upper, p.owned, upper_begin, upper_end, cols, true, shape)) return;
-    if (!build_direction(ctx, p.lower_local, p.owned, p.bs, element_size, element_size, p.lower, lower, upper,
-                         lower_begin, lower_end, cols, false, ssor, shape, shared_rows)
-        || !build_direction(ctx, p.upper_local, p.owned, p.bs, element_size, element_size, p.upper, upper, lower,
-                            upper_begin, upper_end, cols, true, true, shape, shared_rows)) {
+    if (!both([&] { return cut_steps(lower, p.lower, p.owned, lower_begin, lower_end, cols, false, shape); },
+              [&] { return cut_steps(upper, p.upper, p.owned, upper_begin, upper_end, cols, true, shape); })) return;
+    Plan lower_plan, upper_plan;
+    if (!both([&] { return plan_direction(lower_plan, p.lower_local, p.owned, p.lower, lower, upper, lower_begin,
+                                          lower_end, cols, false, shape, shared_rows); },
+              [&] { return plan_direction(upper_plan, p.upper_local, p.owned, p.upper, upper, lower, upper_begin,
+                                          upper_end, cols, true, shape, shared_rows); })) {
         p.lower_local = LocalSweep();
         p.upper_local = LocalSweep();
+        return;
     }
+    place_direction(ctx, p.lower_local, lower_plan, lower, p.bs, element_size, element_size, ssor, shape);
+    place_direction(ctx, p.upper_local, upper_plan, upper, p.bs, element_size, element_size, true, shape);
 }
 
 namespace {
@@ -1033,19 +1061,23 @@ void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage
     std::vector<std::int32_t> after(n);   // first upper entry of each row
     for (std::size_t r = 0; r < n; ++r) after[r] = dp[r] + 1;
     Cut lower, upper;
-    if (!cut_steps(lower, p.lower, n, rp, dp, ci, false, shape)
-        || !cut_steps(upper, p.upper, n, after.data(), rp + 1, ci, true, shape)) return;
+    if (!both([&] { return cut_steps(lower, p.lower, n, rp, dp, ci, false, shape); },
+              [&] { return cut_steps(upper, p.upper, n, after.data(), rp + 1, ci, true, shape); })) return;
     const std::size_t tasks = (lower.task.size() + upper.task.size()) / 4;
     const double task_ns = kBlockTaskNs[storage == OWTK_F64 ? 2 : storage == OWTK_F32 ? 1 : 0][bs - 1];
     const double level_ns = storage == OWTK_F64 ? 1400.0 : 1100.0;
     if (static_cast<double>(tasks) * task_ns > level_ns * (p.lower.depth + p.upper.depth)) return;
-    if (!build_direction(ctx, p.lower_local, n, bs, vector, value, p.lower, lower, upper, rp, dp, ci, false, false, shape,
-                         shared_rows)
-        || !build_direction(ctx, p.upper_local, n, bs, vector, value, p.upper, upper, lower, after.data(), rp + 1, ci,
-                            true, true, shape, shared_rows)) {
+    Plan lower_plan, upper_plan;
+    if (!both([&] { return plan_direction(lower_plan, p.lower_local, n, p.lower, lower, upper, rp, dp, ci, false, shape,
+                                          shared_rows); },
+              [&] { return plan_direction(upper_plan, p.upper_local, n, p.upper, upper, lower, after.data(), rp + 1,
+                                          ci, true, shape, shared_rows); })) {
         p.lower_local = LocalSweep();
         p.upper_local = LocalSweep();
+        return;
     }
+    place_direction(ctx, p.lower_local, lower_plan, lower, bs, vector, value, false, shape);
+    place_direction(ctx, p.upper_local, upper_plan, upper, bs, vector, value, true, shape);
 }
 
 namespace kern {

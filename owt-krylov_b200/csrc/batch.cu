@@ -426,9 +426,13 @@ __device__ void advance(const Args& a, int phase, int sys, const Reduced& r, uns
         atomicMax(&a.grid->checks, cycle + (phase == kEw5 ? 2 : 1));
 }
 
-// Warp-collective: the system's partials combined, its state advanced.
+// Warp-collective, after lane 0's arrival turned out to be the last: the
+// system's partials combined, its state advanced.  The barrier carries lane 0's
+// acquire over to the lanes that load the other segments' partials; the shuffle
+// that told them of it orders no memory.
 __device__ __forceinline__ void finalize(const Args& a, int phase, int sys, unsigned long long cycle)
 {
+    __syncwarp();
     const Sys y = a.sys[sys];
     const Reduced r = phase == kSp1 || phase == kSp2 ? combine_sp(a, y, phase == kSp2) : combine_ew(a, y, phase == kEw0);
     if ((threadIdx.x & 31) == 0) advance(a, phase, sys, r, cycle);

@@ -21,7 +21,7 @@ def test_solves_repeat_bit_for_bit(native, ctx, problems, sides):
     first = None
     for run in range(12):
         x.fill(0.0)
-        results = [r.as_dict() for r in batch.solve(b, x)]
+        results = [{k: v for k, v in r.as_dict().items() if k != "solve_seconds"} for r in batch.solve(b, x)]
         assert results[0]["status"] == 0
         if first is None:
             first = x.download(), results

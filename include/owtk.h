@@ -213,6 +213,26 @@ owtk_status owtk_pc_chain_schedule(owtk_preconditioner* pc, int32_t* windows);
 owtk_status owtk_pc_lockstep_schedule(owtk_preconditioner* pc, int32_t* cluster_ctas, int32_t* lower_levels,
                                       int32_t* upper_levels);
 
+/* One CTA per component, or for dense blocks one CTA (no reference
+ * counterpart): how ILU and SSOR applies run while their levels are narrow.
+ * The same bits as every other schedule. */
+typedef struct owtk_local_schedule {
+    int32_t warps;          /* tasks (of up to 32 rows) per step; 0: another schedule is in use */
+    int32_t lower_steps;    /* forward sweep */
+    int32_t upper_steps;    /* backward sweep */
+    int32_t ring_rows;      /* rows whose results shared memory holds */
+    int32_t far_values;     /* dependencies read from global memory because they lie further back */
+    int32_t slow_tasks;     /* tasks with longer rows, or more far values, than a stage holds */
+    int32_t far_steps;      /* least number of steps that a far value lies back; INT32_MAX without any */
+} owtk_local_schedule;
+/* The schedule that ILU(0) and SSOR applies of this pattern take, computed
+ * without a GPU: element_size 4 or 8 bytes a value, ring_rows 0 for as many as
+ * shared memory holds.  A ring so short that a far value could be copied before
+ * it is written gives no schedule. */
+owtk_status owtk_local_schedule_plan(size_t owned_nodes, size_t block_size, const uint64_t* row_offsets,
+                                     const uint64_t* column_indices, size_t element_size, int32_t ring_rows,
+                                     owtk_local_schedule* out);
+
 /* ---- host setup (ordering.hpp) -------------------------------------------- */
 /* reverse_cuthill_mckee_order (ordering.hpp:138-180); new_to_old[owned]. */
 owtk_status owtk_rcm_order(size_t owned_nodes, size_t ghost_nodes, const uint64_t* row_offsets,

@@ -43,6 +43,7 @@
 // explicit rounding, so results equal the CPU path bit for bit.
 
 #include <algorithm>
+#include <cstdint>
 #include <cstdlib>
 #include <future>
 #include <type_traits>
@@ -758,7 +759,15 @@ struct Cut {
 struct Shape {
     int warps, rows, entries, pad;
     bool block;
+    int teams;
 };
+
+// Steps that a far value must lie back.  The team that takes step s copies its
+// task's far values when it is done with step s - kDepth * teams, whose wait put
+// it behind all that was done before the signal of the step before; a result
+// goes to global memory behind its own step's signal, so before the signal
+// that its team gives `teams` steps later.
+constexpr int far_reach(int teams) { return (kDepth + 1) * teams + 1; }
 
 // Rows by level and row number, cut into tasks and steps.  (Within a level by
 // number of dependencies, for less padding: the same times.)  False for a row
@@ -829,9 +838,15 @@ bool plan_direction(Plan& plan, LocalSweep& s, std::size_t owned, const Sweep& s
     auto far_index = [&](std::int32_t col) { return backward ? col : other.place[col]; };
     std::size_t first = 0, used = 0, slow_tasks = 0;
     std::vector<std::int32_t>& far = plan.far;
+    auto step_of = [&](std::int32_t p) {   // of a place: that of the last task starting at or before it
+        std::size_t a = 0, b = cut.task.size() / 4;
+        while (b - a > 1) (cut.task[(a + b) / 2 * 4 + 1] <= p ? a : b) = (a + b) / 2;
+        return static_cast<std::int32_t>(a) / warps;
+    };
+    s.far_steps = INT32_MAX;
     for (std::size_t t = 0; t < cut.task.size(); t += 4) {
         std::int32_t* w = cut.task.data() + t;
-        const std::int32_t rows = w[2] & 0xff, width = w[2] >> 8;
+        const std::int32_t rows = w[2] & 0xff, width = w[2] >> 8, step = static_cast<std::int32_t>(t / 4) / warps;
         std::size_t found = 0;
         for (std::int32_t p = w[1]; p < w[1] + rows; ++p) {
             const std::int32_t row = cut.rows[p];
@@ -841,8 +856,10 @@ bool plan_direction(Plan& plan, LocalSweep& s, std::size_t owned, const Sweep& s
                 if (far.empty()) far.assign(cut.task.size() / 4 * 32, -1);
                 if (found < 32) far[t / 4 * 32 + found] = far_index(cols[k]);
                 ++found;
+                s.far_steps = std::min(s.far_steps, step - step_of(place[cols[k]]));
             }
         }
+        s.far_values += static_cast<int>(found);
         const bool slow = width > kHold || found > 32;
         if (slow && shape.block) return false;
         w[0] = static_cast<std::int32_t>(first);
@@ -853,6 +870,11 @@ bool plan_direction(Plan& plan, LocalSweep& s, std::size_t owned, const Sweep& s
         if (first >= static_cast<std::size_t>(kMaxEntries)) return false;
     }
     s.entries = first;
+    s.slow_tasks = static_cast<int>(slow_tasks);
+    // A copy could pass the result that it is to bring.  (With the rings that
+    // shared memory holds the closest lie 67 steps back against 28, FP64 blocks
+    // of 3; a ring of few rows, or more tasks in flight, end here.)
+    if (s.far_steps < far_reach(shape.teams)) return false;
     // A few rows much longer than the rest would pad their tasks' other rows.
     if (s.entries > 4 * used + 8 * owned + 4096) return false;
     // A task of the slower form costs its step about a microsecond, more than
@@ -889,6 +911,44 @@ bool plan_direction(Plan& plan, LocalSweep& s, std::size_t owned, const Sweep& s
     return true;
 }
 
+// What both directions of a component-diagonal sweep need, on the host.
+struct Planned {
+    Cut lower, upper;
+    Plan lower_plan, upper_plan;
+};
+
+constexpr int teams_of(int warps) { return warps == 1 ? kTeams1 : warps == 2 ? kTeams2 : kTeams4; }
+Shape component_shape(int warps) { return Shape{warps, 32, kTaskEntries, 4, false, teams_of(warps)}; }
+
+// Both directions side by side, the lower one on another thread where one can
+// be had.
+template<class L, class U> bool both(L lower, U upper)
+{
+    std::future<bool> first = std::async(lower);
+    const bool second = upper();
+    return first.get() && second;
+}
+
+// ring_rows: 0 for as many as shared memory holds.
+bool plan_local(Planned& x, LocalSweep& lo, LocalSweep& up, const Sweep& lower, const Sweep& upper, std::size_t owned,
+                int warps, std::size_t element_size, int ring_rows, const std::int32_t* lower_begin,
+                const std::int32_t* lower_end, const std::int32_t* upper_begin, const std::int32_t* upper_end,
+                const std::int32_t* cols)
+{
+    const Shape shape = component_shape(warps);
+    if (ring_rows == 0) {
+        const std::size_t stage = element_size == 8 ? sizeof(Stage<double>) : sizeof(Stage<float>);
+        const std::size_t stages = static_cast<std::size_t>(warps * shape.teams * kDepth) * stage;
+        ring_rows = static_cast<int>((kSharedBytes - stages) / element_size) - 2;
+    }
+    return both([&] { return cut_steps(x.lower, lower, owned, lower_begin, lower_end, cols, false, shape); },
+                [&] { return cut_steps(x.upper, upper, owned, upper_begin, upper_end, cols, true, shape); })
+        && both([&] { return plan_direction(x.lower_plan, lo, owned, lower, x.lower, x.upper, lower_begin, lower_end,
+                                            cols, false, shape, ring_rows); },
+                [&] { return plan_direction(x.upper_plan, up, owned, upper, x.upper, x.lower, upper_begin, upper_end,
+                                            cols, true, shape, ring_rows); });
+}
+
 // The plan on the device.  vector_size, value_size: bytes of a vector element
 // and of a stored value.
 void place_direction(Context& ctx, LocalSweep& s, const Plan& plan, const Cut& cut, std::size_t bs,
@@ -914,29 +974,18 @@ void place_direction(Context& ctx, LocalSweep& s, const Plan& plan, const Cut& c
     s.ready = true;
 }
 
-// Both directions side by side, the lower one on another thread where one can
-// be had.
-template<class L, class U> bool both(L lower, U upper)
-{
-    std::future<bool> first = std::async(lower);
-    const bool second = upper();
-    return first.get() && second;
-}
-
-constexpr int teams_of(int warps) { return warps == 1 ? kTeams1 : warps == 2 ? kTeams2 : kTeams4; }
-
 }  // namespace
 
 // Warps per team of the cheapest shape, or 0 when the level-scheduled sweep is
 // cheaper: the steps of each shape at their measured cost against 800 ns a
 // level (0.71 to 0.86 us measured at 250 to 1,400 rows a level).  The line lies
 // at about 700 rows a level, where both take 0.8 us.
-int local_sweep_warps(const Context& ctx, const Sweep& lower, const Sweep& upper, std::size_t owned, std::size_t bs)
+int local_sweep_warps(int sm_count, const Sweep& lower, const Sweep& upper, std::size_t owned, std::size_t bs)
 {
     static constexpr struct { int warps; double ns; } kShapes[] = {{1, 75}, {2, 95}, {4, 145}};
     const char* env = std::getenv("OWTK_LOCAL_SWEEP");   // 0: never
     if (env && std::atoi(env) == 0) return 0;
-    if (owned == 0 || bs > static_cast<std::size_t>(ctx.sm_count)) return 0;
+    if (owned == 0 || bs > static_cast<std::size_t>(sm_count)) return 0;
     std::vector<std::size_t> size;
     for (const Sweep* s : {&lower, &upper}) {
         const std::size_t at = size.size();
@@ -963,24 +1012,46 @@ void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t e
                        const std::int32_t* lower_begin, const std::int32_t* lower_end, const std::int32_t* upper_begin,
                        const std::int32_t* upper_end, const std::int32_t* cols, bool ssor)
 {
-    const std::size_t stage = element_size == 8 ? sizeof(Stage<double>) : sizeof(Stage<float>);
-    const int shared_rows =
-        static_cast<int>((kSharedBytes - static_cast<std::size_t>(warps * teams_of(warps) * kDepth) * stage) / element_size) - 2;
-    Cut lower, upper;
-    const Shape shape{warps, 32, kTaskEntries, 4, false};
-    if (!both([&] { return cut_steps(lower, p.lower, p.owned, lower_begin, lower_end, cols, false, shape); },
-              [&] { return cut_steps(upper, p.upper, p.owned, upper_begin, upper_end, cols, true, shape); })) return;
-    Plan lower_plan, upper_plan;
-    if (!both([&] { return plan_direction(lower_plan, p.lower_local, p.owned, p.lower, lower, upper, lower_begin,
-                                          lower_end, cols, false, shape, shared_rows); },
-              [&] { return plan_direction(upper_plan, p.upper_local, p.owned, p.upper, upper, lower, upper_begin,
-                                          upper_end, cols, true, shape, shared_rows); })) {
+    const Shape shape = component_shape(warps);
+    Planned x;
+    if (!plan_local(x, p.lower_local, p.upper_local, p.lower, p.upper, p.owned, warps, element_size, 0, lower_begin,
+                    lower_end, upper_begin, upper_end, cols)) {
         p.lower_local = LocalSweep();
         p.upper_local = LocalSweep();
         return;
     }
-    place_direction(ctx, p.lower_local, lower_plan, lower, p.bs, element_size, element_size, ssor, shape);
-    place_direction(ctx, p.upper_local, upper_plan, upper, p.bs, element_size, element_size, true, shape);
+    place_direction(ctx, p.lower_local, x.lower_plan, x.lower, p.bs, element_size, element_size, ssor, shape);
+    place_direction(ctx, p.upper_local, x.upper_plan, x.upper, p.bs, element_size, element_size, true, shape);
+}
+
+owtk_local_schedule local_schedule(const LocalSweep& lower, const LocalSweep& upper)
+{
+    owtk_local_schedule s{};
+    s.warps = lower.warps;
+    s.lower_steps = lower.steps;
+    s.upper_steps = upper.steps;
+    s.ring_rows = std::min(lower.ring, upper.ring);
+    s.far_values = lower.far_values + upper.far_values;
+    s.slow_tasks = lower.slow_tasks + upper.slow_tasks;
+    s.far_steps = std::min(lower.far_steps, upper.far_steps);
+    return s;
+}
+
+// No CUDA call.
+owtk_local_schedule plan_local_schedule(std::size_t owned, std::size_t bs, const std::int32_t* rowptr,
+                                        const std::int32_t* cols, std::size_t element_size, int sm_count, int ring_rows)
+{
+    std::vector<std::int32_t> lower_level, upper_level;
+    levels_of(owned, rowptr, cols, lower_level, upper_level);
+    Sweep lower, upper;
+    order_by_level(lower, owned, bs, lower_level);
+    order_by_level(upper, owned, bs, upper_level);
+    const int warps = local_sweep_warps(sm_count, lower, upper, owned, bs);
+    LocalSweep lo, up;
+    Planned x;
+    if (warps == 0 || !plan_local(x, lo, up, lower, upper, owned, warps, element_size, ring_rows, rowptr, rowptr + 1,
+                                  rowptr, rowptr + 1, cols)) return {};
+    return local_schedule(lo, up);
 }
 
 namespace {
@@ -1053,8 +1124,8 @@ void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage
                       value = storage == OWTK_F64 ? 8 : storage == OWTK_F32 ? 4 : 2;
     const std::size_t stage = storage == OWTK_F64 ? block_stage_bytes<double, double>(bs)
         : storage == OWTK_F32 ? block_stage_bytes<float, float>(bs) : block_stage_bytes<float, __nv_bfloat16>(bs);
-    const Shape shape{1, 32, block_entries(value * bs * bs), 8, true};
-    const std::size_t stages = block_teams(stage) * kDepth * stage, row = (bs == 3 ? 4 : bs) * vector;
+    const Shape shape{1, 32, block_entries(value * bs * bs), 8, true, block_teams(stage)};
+    const std::size_t stages = shape.teams * kDepth * stage, row = (bs == 3 ? 4 : bs) * vector;
     if (n == 0 || stages + 1024 * row > kSharedBytes) return;
     const int shared_rows = static_cast<int>((kSharedBytes - stages) / row) - 2;
     const std::int32_t *rp = p.f_rowptr.data(), *dp = p.f_diagpos.data(), *ci = p.f_cols.data();

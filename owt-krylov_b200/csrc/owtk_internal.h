@@ -250,6 +250,9 @@ struct LocalSweep {
     int steps = 0;
     int warps = 1;             // tasks per step
     int ring = 0;              // places whose results shared memory holds
+    int far_values = 0;        // dependencies beyond the ring's reach
+    int far_steps = 0;         // least steps that one lies back (INT32_MAX: there are none)
+    int slow_tasks = 0;
     std::size_t entries = 0;   // padded
     std::size_t places = 0;    // padded rows
     DeviceBuffer task;         // int4 per step and warp: first entry, first place, rows and width (and flags), ring slot
@@ -335,6 +338,8 @@ void build_tile_plan(Matrix& m);
 void build_row_slices(Matrix& m);
 void levels_of(std::size_t owned, const std::int32_t* rowptr, const std::int32_t* cols,
                std::vector<std::int32_t>& lower, std::vector<std::int32_t>& upper);
+std::vector<std::int32_t> order_by_level(Sweep& s, std::size_t owned, std::size_t bs,
+                                         const std::vector<std::int32_t>& level);
 void build_sweep(Context& ctx, Sweep& s, std::size_t owned, std::size_t bs,
                  const std::vector<std::int32_t>& level, bool descending_rows);
 void pack_sweep(Context& ctx, Sweep& s, std::size_t bs, std::size_t element_size,
@@ -350,11 +355,14 @@ void build_cluster_sweep(Context& ctx, ClusterSweep& s, std::size_t owned, std::
                          const std::vector<std::int32_t>& level, const std::vector<std::int32_t>& rowptr,
                          const std::vector<std::int32_t>& cols, const std::vector<std::int32_t>& diagpos,
                          bool backward, std::vector<std::uint32_t>& loc);
-int local_sweep_warps(const Context& ctx, const Sweep& lower, const Sweep& upper, std::size_t owned, std::size_t bs);
+int local_sweep_warps(int sm_count, const Sweep& lower, const Sweep& upper, std::size_t owned, std::size_t bs);
 void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t element_size,
                        const std::int32_t* lower_begin, const std::int32_t* lower_end, const std::int32_t* upper_begin,
                        const std::int32_t* upper_end, const std::int32_t* cols, bool ssor);
 void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage);
+owtk_local_schedule local_schedule(const LocalSweep& lower, const LocalSweep& upper);
+owtk_local_schedule plan_local_schedule(std::size_t owned, std::size_t bs, const std::int32_t* rowptr,
+                                        const std::int32_t* cols, std::size_t element_size, int sm_count, int ring_rows);
 void rcm_order(std::size_t owned, const std::int32_t* rowptr, const std::int32_t* cols,
                std::uint64_t* out);
 void hilbert_order(std::size_t n, const double* xy, std::uint64_t* out);

@@ -43,8 +43,8 @@ void levels_of(std::size_t owned, const std::int32_t* rowptr, const std::int32_t
 
 // Rows bucketed by level (ascending rows inside a level), cut into tasks of
 // at most rows_per_task rows that never cross a level boundary.
-void build_sweep(Context& ctx, Sweep& s, std::size_t owned, std::size_t bs,
-                 const std::vector<std::int32_t>& level, bool /*descending_rows*/)
+std::vector<std::int32_t> order_by_level(Sweep& s, std::size_t owned, std::size_t bs,
+                                         const std::vector<std::int32_t>& level)
 {
     s.h_level = level;
     s.rows_per_task = bs <= 32 ? static_cast<int>(32 / bs) : 1;
@@ -69,9 +69,16 @@ void build_sweep(Context& ctx, Sweep& s, std::size_t owned, std::size_t bs,
         }
     }
     s.tasks = static_cast<int>(tasks.size()) - 1;
-    s.order = upload(ctx.stream, order);
-    s.task_start = upload(ctx.stream, tasks);
     s.h_order = std::move(order);
+    return tasks;
+}
+
+void build_sweep(Context& ctx, Sweep& s, std::size_t owned, std::size_t bs,
+                 const std::vector<std::int32_t>& level, bool /*descending_rows*/)
+{
+    const std::vector<std::int32_t> tasks = order_by_level(s, owned, bs, level);
+    s.order = upload(ctx.stream, s.h_order);
+    s.task_start = upload(ctx.stream, tasks);
 }
 
 // The factor entries an ILU sweep reads (lower entries for the forward sweep,

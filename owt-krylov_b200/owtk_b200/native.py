@@ -74,6 +74,11 @@ class BatchSystem(ctypes.Structure):
                 ("values", c_void_p)]
 
 
+class LocalSchedule(ctypes.Structure):
+    _fields_ = [(name, c_int32) for name in ("warps", "lower_steps", "upper_steps", "ring_rows", "far_values",
+                                             "slow_tasks", "far_steps")]
+
+
 _lib = None
 
 
@@ -128,6 +133,7 @@ def lib():
             "owtk_hilbert_order": (c_int, [sz, vp, vp]),
             "owtk_inverse_permutation": (c_int, [sz, vp, vp]),
             "owtk_level_sets": (c_int, [sz, vp, vp, vp, vp, u64p, u64p]),
+            "owtk_local_schedule_plan": (c_int, [sz, sz, vp, vp, sz, c_int32, POINTER(LocalSchedule)]),
             "owtk_default_options": (None, [POINTER(SolverOptions)]),
             "owtk_workspace_create": (c_int, [vp, POINTER(vp)]),
             "owtk_workspace_destroy": (c_int, [vp]),
@@ -465,6 +471,14 @@ class Preconditioner:
         dl, du = c_uint64(), c_uint64()
         check(lib().owtk_pc_levels(self.h, _ptr(lo), _ptr(up), ctypes.byref(dl), ctypes.byref(du)))
         return lo, up, dl.value, du.value
+
+
+def local_schedule_plan(owned: int, bs: int, rowptr, cols, element_size: int = 8, ring_rows: int = 0) -> LocalSchedule:
+    """The one-CTA-per-component schedule of a pattern's ILU(0) and SSOR applies (warps 0: another one), on the host."""
+    rp, ci = _u64(rowptr), _u64(cols)
+    out = LocalSchedule()
+    check(lib().owtk_local_schedule_plan(owned, bs, _ptr(rp), _ptr(ci), element_size, ring_rows, ctypes.byref(out)))
+    return out
 
     def close(self):
         if self.h is not None:

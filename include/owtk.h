@@ -225,6 +225,8 @@ typedef struct owtk_local_schedule {
     int32_t slow_tasks;     /* tasks with longer rows, or more far values, than a stage holds */
     int32_t far_steps;      /* least number of steps that a far value lies back; INT32_MAX without any */
 } owtk_local_schedule;
+/* The schedule that an ILU, SSOR or block ILU preconditioner's applies run on. */
+owtk_status owtk_pc_local_schedule(owtk_preconditioner* pc, owtk_local_schedule* out);
 /* The schedule that ILU(0) and SSOR applies of this pattern take, computed
  * without a GPU: element_size 4 or 8 bytes a value, ring_rows 0 for as many as
  * shared memory holds.  A ring so short that a far value could be copied before

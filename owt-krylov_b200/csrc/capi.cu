@@ -1553,6 +1553,14 @@ owtk_status owtk_pc_chain_schedule(owtk_preconditioner* pc, int32_t* windows)
     });
 }
 
+owtk_status owtk_pc_local_schedule(owtk_preconditioner* pc, owtk_local_schedule* out)
+{
+    return guarded([&] {
+        require(pc != nullptr && out != nullptr, "null handle");
+        *out = pc->upper_local.ready ? local_schedule(pc->lower_local, pc->upper_local) : owtk_local_schedule{};
+    });
+}
+
 // ------------------------------------------------------------ bounded waits
 owtk_status owtk_debug_unpublished_dependency(owtk_context* ctx, uint32_t spin_limit)
 {

@@ -133,6 +133,7 @@ def lib():
             "owtk_hilbert_order": (c_int, [sz, vp, vp]),
             "owtk_inverse_permutation": (c_int, [sz, vp, vp]),
             "owtk_level_sets": (c_int, [sz, vp, vp, vp, vp, u64p, u64p]),
+            "owtk_pc_local_schedule": (c_int, [vp, POINTER(LocalSchedule)]),
             "owtk_local_schedule_plan": (c_int, [sz, sz, vp, vp, sz, c_int32, POINTER(LocalSchedule)]),
             "owtk_default_options": (None, [POINTER(SolverOptions)]),
             "owtk_workspace_create": (c_int, [vp, POINTER(vp)]),
@@ -463,6 +464,12 @@ class Preconditioner:
         w = c_int32()
         check(lib().owtk_pc_chain_schedule(self.h, ctypes.byref(w)))
         return w.value
+
+    def local_schedule(self) -> LocalSchedule:
+        """The schedule with one CTA per component (warps 0: the applies take another sweep)."""
+        out = LocalSchedule()
+        check(lib().owtk_pc_local_schedule(self.h, ctypes.byref(out)))
+        return out
 
     def levels(self):
         m = self.matrix

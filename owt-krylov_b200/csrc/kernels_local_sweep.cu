@@ -46,7 +46,9 @@
 #include <cstdint>
 #include <cstdlib>
 #include <future>
+#include <memory>
 #include <type_traits>
+#include <utility>
 
 #include <cuda_bf16.h>
 
@@ -745,13 +747,56 @@ void launch(Context& c, Preconditioner& p, T* out)
     }
 }
 
+// [0, n) in ranges on up to four threads (each direction has its own four), the
+// last one here; below `grain` a range is not worth a thread.
+template<class F> void over_ranges(std::size_t n, std::size_t grain, F f)
+{
+    const std::size_t parts = std::min<std::size_t>(4, n / grain + 1);
+    std::vector<std::future<void>> others;
+    for (std::size_t k = 0; k + 1 < parts; ++k)
+        others.push_back(std::async([&f, n, parts, k] { f(k, n * k / parts, n * (k + 1) / parts); }));
+    f(parts - 1, n * (parts - 1) / parts, n);
+    for (auto& o : others) o.get();
+}
+
+// Both directions side by side, the lower one on another thread where the rows
+// are worth it and one can be had.
+constexpr std::size_t kGrain = 4096;
+template<class L, class U> bool both(std::size_t owned, L lower, U upper)
+{
+    if (owned < kGrain) return lower() && upper();
+    std::future<bool> first = std::async(lower);
+    const bool second = upper();
+    return first.get() && second;
+}
+
+// Entries that the threads fill: not set to anything before.
+template<class T> struct Table {
+    std::unique_ptr<T[]> data;
+    std::size_t size = 0;
+    void allocate(std::size_t n)
+    {
+        data.reset(new T[n]);
+        size = n;
+    }
+    T& operator[](std::size_t i) { return data[i]; }
+};
+
+template<class T> DeviceBuffer upload_table(cudaStream_t stream, const Table<T>& host)
+{
+    DeviceBuffer b(host.size * sizeof(T) + 16);
+    if (host.size > 0)
+        OWTK_CUDA(cudaMemcpyAsync(b.ptr, host.data.get(), host.size * sizeof(T), cudaMemcpyHostToDevice, stream));
+    return b;
+}
+
 // A direction's rows in step order, padded: each task starts at a multiple of
 // four places.
 struct Cut {
     std::vector<std::int32_t> task;    // per step and warp: first entry, first place, rows and width, first ring slot
     std::vector<std::int32_t> rows;    // per place (-1: padding)
-    std::vector<std::int32_t> place;   // per row
-    std::vector<std::int32_t> count;   // dependencies per row
+    Table<std::int32_t> place;         // per row
+    Table<std::int32_t> count;         // dependencies per row
 };
 
 // What a task holds: rows, padded entries, and the multiple its places are
@@ -776,12 +821,20 @@ bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32
                const std::int32_t* cols, bool backward, const Shape& shape)
 {
     const auto n = static_cast<std::int32_t>(owned);
-    cut.count.assign(owned, 0);
-    for (std::int32_t r = 0; r < n; ++r)
-        for (std::int32_t e = begin[r]; e < end[r]; ++e)
-            cut.count[r] += backward ? cols[e] > r && cols[e] < n : cols[e] < r;
+    cut.count.allocate(owned);
+    cut.place.allocate(owned);
+    over_ranges(owned, 8 * kGrain, [&](std::size_t, std::size_t r0, std::size_t r1) {
+        for (auto r = static_cast<std::int32_t>(r0); r < static_cast<std::int32_t>(r1); ++r) {
+            std::int32_t count = 0;
+            for (std::int32_t e = begin[r]; e < end[r]; ++e)
+                count += backward ? cols[e] > r && cols[e] < n : cols[e] < r;
+            cut.count[r] = count;
+        }
+    });
     const std::vector<std::int32_t>&order = sweep.h_order, &level = sweep.h_level;
-    cut.place.resize(owned);
+    const std::size_t steps = owned / static_cast<std::size_t>(shape.warps * shape.rows) + sweep.depth;
+    cut.task.reserve(4 * shape.warps * steps);
+    cut.rows.reserve(owned + static_cast<std::size_t>(shape.pad) * shape.warps * steps);
     std::int32_t at = 0;
     for (std::int32_t b = 0; b < n;) {
         std::int32_t e = b;
@@ -798,12 +851,11 @@ bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32
                 }
                 if (width > 0xff) return false;
                 cut.task.insert(cut.task.end(), {0, at, rows | width << 8, 0});
-                for (std::int32_t l = 0; l < rows; ++l) {
-                    cut.place[order[b + l]] = at + l;
-                    cut.rows.push_back(order[b + l]);
-                }
-                while (cut.rows.size() % shape.pad != 0) cut.rows.push_back(-1);
-                at = static_cast<std::int32_t>(cut.rows.size());
+                for (std::int32_t l = 0; l < rows; ++l) cut.place[order[b + l]] = at + l;
+                const std::int32_t padded = (rows + shape.pad - 1) / shape.pad * shape.pad;
+                cut.rows.insert(cut.rows.end(), order.begin() + b, order.begin() + b + rows);
+                cut.rows.insert(cut.rows.end(), static_cast<std::size_t>(padded - rows), -1);
+                at += padded;
                 b += rows;
             }
         }
@@ -814,8 +866,9 @@ bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32
 
 // A direction's tables on the host.
 struct Plan {
-    std::vector<std::int32_t> far, code, src, to;
-    std::vector<std::uint16_t> slots;
+    std::vector<std::int32_t> far, code;
+    Table<std::int32_t> src, to;
+    Table<std::uint16_t> slots;
 };
 
 // Fills the sizes of s, the tasks of cut and the plan; false where the
@@ -827,86 +880,120 @@ bool plan_direction(Plan& plan, LocalSweep& s, std::size_t owned, const Sweep& s
 {
     const int warps = shape.warps;
     const auto n = static_cast<std::int32_t>(owned);
-    const std::vector<std::int32_t>& place = cut.place;
+    const std::size_t tasks = cut.task.size() / 4;
+    const std::int32_t* place = cut.place.data.get();
     s.warps = warps;
     s.places = cut.rows.size();
-    s.steps = static_cast<int>(cut.task.size() / 4) / warps;
+    s.steps = static_cast<int>(tasks) / warps;
     s.ring = std::min(static_cast<std::int32_t>(s.places), std::min(shared_rows, kFarSlot - 1));
     // A step's results may not overwrite what the same step still reads.
     const std::int32_t reach = static_cast<std::int32_t>(s.places) > s.ring ? s.ring - 32 * warps : s.ring;
     auto needed = [&](std::int32_t row, std::int32_t col) { return backward ? col > row && col < n : col < row; };
-    auto far_index = [&](std::int32_t col) { return backward ? col : other.place[col]; };
-    std::size_t first = 0, used = 0, slow_tasks = 0;
-    std::vector<std::int32_t>& far = plan.far;
-    auto step_of = [&](std::int32_t p) {   // of a place: that of the last task starting at or before it
-        std::size_t a = 0, b = cut.task.size() / 4;
-        while (b - a > 1) (cut.task[(a + b) / 2 * 4 + 1] <= p ? a : b) = (a + b) / 2;
-        return static_cast<std::int32_t>(a) / warps;
-    };
-    s.far_steps = INT32_MAX;
-    for (std::size_t t = 0; t < cut.task.size(); t += 4) {
-        std::int32_t* w = cut.task.data() + t;
-        const std::int32_t rows = w[2] & 0xff, width = w[2] >> 8, step = static_cast<std::int32_t>(t / 4) / warps;
-        std::size_t found = 0;
-        for (std::int32_t p = w[1]; p < w[1] + rows; ++p) {
-            const std::int32_t row = cut.rows[p];
-            used += static_cast<std::size_t>(cut.count[row]);
-            for (std::int32_t k = begin[row]; k < end[row]; ++k) {
-                if (!needed(row, cols[k]) || p - place[cols[k]] <= reach) continue;
-                if (far.empty()) far.assign(cut.task.size() / 4 * 32, -1);
-                if (found < 32) far[t / 4 * 32 + found] = far_index(cols[k]);
-                ++found;
-                s.far_steps = std::min(s.far_steps, step - step_of(place[cols[k]]));
-            }
-        }
-        s.far_values += static_cast<int>(found);
-        const bool slow = width > kHold || found > 32;
-        if (slow && shape.block) return false;
+    auto far_index = [&](std::int32_t col) { return backward ? col : other.place.data[col]; };
+    std::size_t first = 0, used = 0;
+    for (std::size_t r = 0; r < owned; ++r) used += static_cast<std::size_t>(cut.count[r]);
+    for (std::size_t t = 0; t < tasks; ++t) {
+        std::int32_t* w = cut.task.data() + 4 * t;
         w[0] = static_cast<std::int32_t>(first);
-        w[2] |= slow ? kSlowFlag : found > 0 ? kFarFlag : 0;
         w[3] = w[1] % s.ring;
-        first += (static_cast<std::size_t>(rows) * width + 7) / 8 * 8;
-        slow_tasks += slow;
+        first += (static_cast<std::size_t>(w[2] & 0xff) * (w[2] >> 8) + 7) / 8 * 8;
         if (first >= static_cast<std::size_t>(kMaxEntries)) return false;
     }
     s.entries = first;
+    // A few rows much longer than the rest would pad their tasks' other rows.
+    if (s.entries > 4 * used + 8 * owned + 4096) return false;
+
+    plan.src.allocate(s.entries);
+    plan.slots.allocate(s.entries);
+    auto step_of = [&](std::int32_t p) {   // of a place: that of the last task starting at or before it
+        std::size_t a = 0, b = tasks;
+        while (b - a > 1) (cut.task[(a + b) / 2 * 4 + 1] <= p ? a : b) = (a + b) / 2;
+        return static_cast<std::int32_t>(a) / warps;
+    };
+    struct Part {
+        std::vector<std::pair<std::size_t, std::int32_t>> far;   // where in plan.far, and what
+        std::size_t far_values = 0, slow_tasks = 0;
+        int far_steps = INT32_MAX;
+    } parts[4];
+    over_ranges(tasks, kGrain / 8, [&](std::size_t part, std::size_t t0, std::size_t t1) {
+        Part& out = parts[part];
+        for (std::size_t t = t0; t < t1; ++t) {
+            std::int32_t* w = cut.task.data() + 4 * t;
+            const std::int32_t rows = w[2] & 0xff, width = w[2] >> 8;
+            std::int32_t* src = plan.src.data.get() + w[0];
+            std::uint16_t* slots = plan.slots.data.get() + w[0];
+            std::size_t found = 0;
+            for (std::int32_t l = 0; l < rows; ++l) {
+                const std::int32_t p = w[1] + l, row = cut.rows[p], own = w[3] + l < s.ring ? w[3] + l : w[3] + l - s.ring;
+                auto set = [&](std::int32_t j, std::int32_t slot, std::int32_t entry) {
+                    slots[shape.block ? j * rows + l : (j & ~1) * rows + 2 * l + j % 2] = static_cast<std::uint16_t>(slot);
+                    src[j * rows + l] = entry;
+                };
+                std::int32_t j = 0;
+                for (std::int32_t e = begin[row]; e < end[row]; ++e) {
+                    if (!needed(row, cols[e])) continue;
+                    const std::int32_t back = p - place[cols[e]];
+                    if (back <= reach) {
+                        set(j++, back <= own ? own - back : own - back + s.ring, e);
+                        continue;
+                    }
+                    if (found < 32) out.far.emplace_back(t * 32 + found, far_index(cols[e]));
+                    set(j++, kFarSlot + static_cast<std::int32_t>(found++ % 32), e);
+                    out.far_steps = std::min(out.far_steps, static_cast<std::int32_t>(t) / warps - step_of(p - back));
+                }
+                for (; j < width; ++j) set(j, s.ring, -1);
+            }
+            for (std::int32_t i = rows * width; i % 8 != 0; ++i) {
+                slots[i] = static_cast<std::uint16_t>(s.ring);
+                src[i] = -1;
+            }
+            const bool slow = width > kHold || found > 32;
+            w[2] |= slow ? kSlowFlag : found > 0 ? kFarFlag : 0;
+            out.far_values += found;
+            out.slow_tasks += slow;
+        }
+    });
+    std::size_t far_values = 0, slow_tasks = 0;
+    s.far_steps = INT32_MAX;
+    for (const Part& part : parts) {
+        far_values += part.far_values;
+        slow_tasks += part.slow_tasks;
+        s.far_steps = std::min(s.far_steps, part.far_steps);
+    }
+    s.far_values = static_cast<int>(far_values);
     s.slow_tasks = static_cast<int>(slow_tasks);
+    if (slow_tasks > 0 && shape.block) return false;
     // A copy could pass the result that it is to bring.  (With the rings that
     // shared memory holds the closest lie 67 steps back against 28, FP64 blocks
     // of 3; a ring of few rows, or more tasks in flight, end here.)
     if (s.far_steps < far_reach(shape.teams)) return false;
-    // A few rows much longer than the rest would pad their tasks' other rows.
-    if (s.entries > 4 * used + 8 * owned + 4096) return false;
     // A task of the slower form costs its step about a microsecond, more than
     // a level of the level-scheduled sweep.
     if (slow_tasks > static_cast<std::size_t>(sweep.depth) / 4) return false;
-    const bool any_slow = slow_tasks > 0;
-    plan.code.assign(any_slow ? s.entries : 0, s.ring);
-    plan.src.assign(s.entries, -1);
-    plan.slots.assign(s.entries, static_cast<std::uint16_t>(s.ring));
-    for (std::size_t t = 0; t < cut.task.size(); t += 4) {
-        const std::size_t base = static_cast<std::size_t>(cut.task[t]), rows = cut.task[t + 2] & 0xff;
-        std::size_t found = 0;
-        for (std::size_t l = 0; l < rows; ++l) {
-            const std::int32_t p = cut.task[t + 1] + static_cast<std::int32_t>(l), row = cut.rows[p];
-            std::size_t j = 0;
-            for (std::int32_t e = begin[row]; e < end[row]; ++e) {
-                if (!needed(row, cols[e])) continue;
-                const std::int32_t from = place[cols[e]];
-                const bool near = p - from <= reach;
-                const std::size_t slot = near ? from % s.ring : kFarSlot + found++ % 32;
-                plan.slots[shape.block ? base + j * rows + l : base + (j & ~std::size_t(1)) * rows + 2 * l + j % 2] =
-                    static_cast<std::uint16_t>(slot);
-                if (any_slow) plan.code[base + j * rows + l] = near ? from % s.ring : -1 - far_index(cols[e]);
-                plan.src[base + j * rows + l] = e;
-                ++j;
+    if (far_values > 0) plan.far.assign(tasks * 32, -1);
+    for (const Part& part : parts)
+        for (const auto& [at, value] : part.far) plan.far[at] = value;
+    if (slow_tasks > 0) {
+        // Every task's dependencies as the slower form reads them.
+        plan.code.assign(s.entries, s.ring);
+        for (std::size_t t = 0; t < tasks; ++t) {
+            const std::int32_t* w = cut.task.data() + 4 * t;
+            const std::int32_t rows = w[2] & 0xff;
+            for (std::int32_t l = 0; l < rows; ++l) {
+                const std::int32_t p = w[1] + l;
+                for (std::int32_t k = w[0] + l; k < w[0] + rows * (w[2] >> 8 & 0xff); k += rows) {
+                    if (plan.src[k] < 0) break;
+                    const std::int32_t col = cols[plan.src[k]], from = place[col];
+                    plan.code[k] = p - from <= reach ? from % s.ring : -1 - far_index(col);
+                }
             }
         }
     }
     if (!backward) {
-        plan.to.assign(s.places, 0);
-        for (std::size_t p = 0; p < s.places; ++p)
-            if (cut.rows[p] >= 0) plan.to[p] = other.place[cut.rows[p]];
+        plan.to.allocate(s.places);
+        over_ranges(s.places, 16 * kGrain, [&](std::size_t, std::size_t p0, std::size_t p1) {
+            for (std::size_t p = p0; p < p1; ++p) plan.to[p] = cut.rows[p] >= 0 ? other.place.data[cut.rows[p]] : 0;
+        });
     }
     return true;
 }
@@ -920,15 +1007,6 @@ struct Planned {
 constexpr int teams_of(int warps) { return warps == 1 ? kTeams1 : warps == 2 ? kTeams2 : kTeams4; }
 Shape component_shape(int warps) { return Shape{warps, 32, kTaskEntries, 4, false, teams_of(warps)}; }
 
-// Both directions side by side, the lower one on another thread where one can
-// be had.
-template<class L, class U> bool both(L lower, U upper)
-{
-    std::future<bool> first = std::async(lower);
-    const bool second = upper();
-    return first.get() && second;
-}
-
 // ring_rows: 0 for as many as shared memory holds.
 bool plan_local(Planned& x, LocalSweep& lo, LocalSweep& up, const Sweep& lower, const Sweep& upper, std::size_t owned,
                 int warps, std::size_t element_size, int ring_rows, const std::int32_t* lower_begin,
@@ -941,9 +1019,9 @@ bool plan_local(Planned& x, LocalSweep& lo, LocalSweep& up, const Sweep& lower, 
         const std::size_t stages = static_cast<std::size_t>(warps * shape.teams * kDepth) * stage;
         ring_rows = static_cast<int>((kSharedBytes - stages) / element_size) - 2;
     }
-    return both([&] { return cut_steps(x.lower, lower, owned, lower_begin, lower_end, cols, false, shape); },
+    return both(owned, [&] { return cut_steps(x.lower, lower, owned, lower_begin, lower_end, cols, false, shape); },
                 [&] { return cut_steps(x.upper, upper, owned, upper_begin, upper_end, cols, true, shape); })
-        && both([&] { return plan_direction(x.lower_plan, lo, owned, lower, x.lower, x.upper, lower_begin, lower_end,
+        && both(owned, [&] { return plan_direction(x.lower_plan, lo, owned, lower, x.lower, x.upper, lower_begin, lower_end,
                                             cols, false, shape, ring_rows); },
                 [&] { return plan_direction(x.upper_plan, up, owned, upper, x.upper, x.lower, upper_begin, upper_end,
                                             cols, true, shape, ring_rows); });
@@ -955,12 +1033,12 @@ void place_direction(Context& ctx, LocalSweep& s, const Plan& plan, const Cut& c
                      std::size_t vector_size, std::size_t value_size, bool with_fin, const Shape& shape)
 {
     s.task = upload(ctx.stream, cut.task);
-    s.slots = upload(ctx.stream, plan.slots);
+    s.slots = upload_table(ctx.stream, plan.slots);
     if (!plan.far.empty()) s.far = upload(ctx.stream, plan.far);
     if (!plan.code.empty()) s.code = upload(ctx.stream, plan.code);
-    s.src = upload(ctx.stream, plan.src);
+    s.src = upload_table(ctx.stream, plan.src);
     s.rows = upload(ctx.stream, cut.rows);
-    s.to = upload(ctx.stream, plan.to);
+    s.to = upload_table(ctx.stream, plan.to);
     // Values of an entry, and of a row's diagonal.
     const std::size_t per = !shape.block ? bs : value_size == 2 ? (bs * bs + 1) / 2 * 2 : bs * bs;
     s.coef.allocate(per * s.entries * value_size + 16);
@@ -1132,14 +1210,14 @@ void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage
     std::vector<std::int32_t> after(n);   // first upper entry of each row
     for (std::size_t r = 0; r < n; ++r) after[r] = dp[r] + 1;
     Cut lower, upper;
-    if (!both([&] { return cut_steps(lower, p.lower, n, rp, dp, ci, false, shape); },
+    if (!both(n, [&] { return cut_steps(lower, p.lower, n, rp, dp, ci, false, shape); },
               [&] { return cut_steps(upper, p.upper, n, after.data(), rp + 1, ci, true, shape); })) return;
     const std::size_t tasks = (lower.task.size() + upper.task.size()) / 4;
     const double task_ns = kBlockTaskNs[storage == OWTK_F64 ? 2 : storage == OWTK_F32 ? 1 : 0][bs - 1];
     const double level_ns = storage == OWTK_F64 ? 1400.0 : 1100.0;
     if (static_cast<double>(tasks) * task_ns > level_ns * (p.lower.depth + p.upper.depth)) return;
     Plan lower_plan, upper_plan;
-    if (!both([&] { return plan_direction(lower_plan, p.lower_local, n, p.lower, lower, upper, rp, dp, ci, false, shape,
+    if (!both(n, [&] { return plan_direction(lower_plan, p.lower_local, n, p.lower, lower, upper, rp, dp, ci, false, shape,
                                           shared_rows); },
               [&] { return plan_direction(upper_plan, p.upper_local, n, p.upper, upper, lower, after.data(), rp + 1,
                                           ci, true, shape, shared_rows); })) {

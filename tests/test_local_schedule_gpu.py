@@ -68,6 +68,18 @@ def test_beyond_the_ring(native, ctx, restatement, kind, width, depth, far, slow
     assert_bitwise(_apply(native, ctx, p, n, 2, x), _want(restatement, kind, n, 2, rp, ci, v, x), kind)
 
 
+# The tables of a direction are filled by up to four threads, from 512 tasks on.
+@pytest.mark.parametrize("kind", ["ilu", "ssor"])
+@pytest.mark.parametrize("width,depth,far", [(24, 600, 0), (60, 1200, 2), (60, 1200, 40)])
+def test_tables_filled_in_ranges(native, ctx, restatement, kind, width, depth, far):
+    n, rp, ci, v = _levels(width, depth, 1, far, far, depth // 3)
+    _, p = _preconditioner(native, ctx, kind, n, 1, rp, ci, v)
+    s = p.local_schedule()
+    assert s.warps > 0 and (s.far_values > 0) == (far > 0) and (s.slow_tasks > 0) == (far > 8)
+    x = np.random.default_rng(5).uniform(-1, 1, n)
+    assert_bitwise(_apply(native, ctx, p, n, 1, x), _want(restatement, kind, n, 1, rp, ci, v, x), kind)
+
+
 @pytest.mark.parametrize("kind", ["ilu", "ssor"])
 @pytest.mark.parametrize("width,slow", [(8, False), (9, True), (17, True)])
 def test_long_rows(native, ctx, restatement, kind, width, slow):

@@ -227,13 +227,13 @@ typedef struct owtk_local_schedule {
 } owtk_local_schedule;
 /* The schedule that an ILU, SSOR or block ILU preconditioner's applies run on. */
 owtk_status owtk_pc_local_schedule(owtk_preconditioner* pc, owtk_local_schedule* out);
-/* The schedule that ILU(0) and SSOR applies of this pattern take, computed
- * without a GPU: element_size 4 or 8 bytes a value, ring_rows 0 for as many as
+/* The schedule that ILU(0) or (ssor != 0) SSOR applies of this pattern take,
+ * computed without a GPU: element_size 4 or 8 bytes a value, ring_rows 0 for as many as
  * shared memory holds.  A ring so short that a far value could be copied before
  * it is written gives no schedule. */
 owtk_status owtk_local_schedule_plan(size_t owned_nodes, size_t block_size, const uint64_t* row_offsets,
-                                     const uint64_t* column_indices, size_t element_size, int32_t ring_rows,
-                                     owtk_local_schedule* out);
+                                     const uint64_t* column_indices, size_t element_size, int32_t ssor,
+                                     int32_t ring_rows, owtk_local_schedule* out);
 
 /* ---- host setup (ordering.hpp) -------------------------------------------- */
 /* reverse_cuthill_mckee_order (ordering.hpp:138-180); new_to_old[owned]. */

@@ -1041,10 +1041,8 @@ std::unique_ptr<owtk_preconditioner> make_pc(owtk_matrix* m, owtk_pc_kind kind, 
         levels_of(m->owned, m->h_rowptr.data(), cols.data(), lower, upper);
         build_sweep(*p->ctx, p->lower, m->owned, m->bs, lower, false);
         build_sweep(*p->ctx, p->upper, m->owned, m->bs, upper, true);
-        if (const int warps = local_sweep_warps(p->ctx->sm_count, p->lower, p->upper, m->owned, m->bs)) {
-            const std::int32_t* rp = m->h_rowptr.data();
-            build_local_sweep(*p->ctx, *p, warps, es, rp, rp + 1, rp, rp + 1, cols.data(), true);
-        }
+        const std::int32_t* rp = m->h_rowptr.data();
+        build_local_sweep(*p->ctx, *p, es, rp, rp + 1, rp, rp + 1, cols.data(), true);
         break;
     }
     case OWTK_PC_ILU: {
@@ -1054,10 +1052,10 @@ std::unique_ptr<owtk_preconditioner> make_pc(owtk_matrix* m, owtk_pc_kind kind, 
         const char* env = std::getenv("OWTK_PACKED_SWEEP");   // 0: applies read the factor in place
         const bool in_place = env && std::atoi(env) == 0;
         const bool scheduled = in_place || p->chain.ready || p->l_lower.ready || p->c_lower.ready;
-        if (const int warps = scheduled ? 0 : local_sweep_warps(p->ctx->sm_count, p->lower, p->upper, m->owned, m->bs)) {
+        if (!scheduled) {
             const std::size_t ls = storage == OWTK_F64 ? es : sizeof(float);
             const std::int32_t *rp = p->f_rowptr.data(), *dp = p->f_diagpos.data(), *ci = p->f_cols.data();
-            build_local_sweep(*p->ctx, *p, warps, ls, rp, dp, dp, rp + 1, ci, false);
+            build_local_sweep(*p->ctx, *p, ls, rp, dp, dp, rp + 1, ci, false);
         }
         if (storage == OWTK_F64 && m->bs <= 32 && !p->chain.ready && !p->upper_local.ready) {
             if (!in_place) {
@@ -1361,7 +1359,7 @@ owtk_status owtk_level_sets(size_t owned, const uint64_t* rowptr, const uint64_t
 }
 
 owtk_status owtk_local_schedule_plan(size_t owned, size_t bs, const uint64_t* rowptr, const uint64_t* cols,
-                                     size_t element_size, int32_t ring_rows, owtk_local_schedule* out)
+                                     size_t element_size, int32_t ssor, int32_t ring_rows, owtk_local_schedule* out)
 {
     return guarded([&] {
         require(out != nullptr, "null output");
@@ -1371,7 +1369,8 @@ owtk_status owtk_local_schedule_plan(size_t owned, size_t bs, const uint64_t* ro
         narrow_pattern(owned, std::numeric_limits<std::int32_t>::max() / 2 - owned, rowptr, cols, rp, ci);
         for (auto& c : ci)
             if (static_cast<std::size_t>(c) >= owned) c = static_cast<std::int32_t>(owned);
-        *out = plan_local_schedule(owned, bs, rp.data(), ci.data(), element_size, 148, ring_rows);
+        *out = plan_local_schedule(owned, bs, rp.data(), ci.data(), element_size, 148, ring_rows,
+                                   ssor != 0);
     });
 }
 

@@ -43,6 +43,7 @@
 // explicit rounding, so results equal the CPU path bit for bit.
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdlib>
 #include <future>
@@ -793,6 +794,11 @@ template<class T> DeviceBuffer upload_table(cudaStream_t stream, const Table<T>&
 // A direction's rows in step order, padded: each task starts at a multiple of
 // four places.
 struct Cut {
+    struct Piece {
+        std::int32_t first, rows, width;   // rows of one level in the sweep's order; their padded dependencies
+        bool ends;                         // the last of its level
+    };
+    std::vector<Piece> pieces;
     std::vector<std::int32_t> task;    // per step and warp: first entry, first place, rows and width, first ring slot
     std::vector<std::int32_t> rows;    // per place (-1: padding)
     Table<std::int32_t> place;         // per row
@@ -814,15 +820,13 @@ struct Shape {
 // that its team gives `teams` steps later.
 constexpr int far_reach(int teams) { return (kDepth + 1) * teams + 1; }
 
-// Rows by level and row number, cut into tasks and steps.  (Within a level by
-// number of dependencies, for less padding: the same times.)  False for a row
-// of more dependencies than a task's width holds.
-bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32_t* begin, const std::int32_t* end,
-               const std::int32_t* cols, bool backward, const Shape& shape)
+// Dependencies of every row: entries [begin, end) with a column below it, or
+// for the backward sweep above it.
+bool count_dependencies(Cut& cut, std::size_t owned, const std::int32_t* begin, const std::int32_t* end,
+                        const std::int32_t* cols, bool backward)
 {
     const auto n = static_cast<std::int32_t>(owned);
     cut.count.allocate(owned);
-    cut.place.allocate(owned);
     over_ranges(owned, 8 * kGrain, [&](std::size_t, std::size_t r0, std::size_t r1) {
         for (auto r = static_cast<std::int32_t>(r0); r < static_cast<std::int32_t>(r1); ++r) {
             std::int32_t count = 0;
@@ -831,37 +835,59 @@ bool cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const std::int32
             cut.count[r] = count;
         }
     });
+    return true;
+}
+
+// Rows by level and row number, cut into tasks.  (Within a level by number of
+// dependencies, for less padding: the same times.)  False for a row of more
+// dependencies than a task's width holds.
+bool cut_tasks(Cut& cut, const Sweep& sweep, std::size_t owned, const Shape& shape)
+{
+    const auto n = static_cast<std::int32_t>(owned);
     const std::vector<std::int32_t>&order = sweep.h_order, &level = sweep.h_level;
-    const std::size_t steps = owned / static_cast<std::size_t>(shape.warps * shape.rows) + sweep.depth;
-    cut.task.reserve(4 * shape.warps * steps);
-    cut.rows.reserve(owned + static_cast<std::size_t>(shape.pad) * shape.warps * steps);
-    std::int32_t at = 0;
+    cut.pieces.reserve(owned / static_cast<std::size_t>(shape.rows) + sweep.depth);
     for (std::int32_t b = 0; b < n;) {
         std::int32_t e = b;
         while (e < n && level[order[e]] == level[order[b]]) ++e;
         while (b < e) {
-            for (int w = 0; w < shape.warps; ++w) {
-                // As many rows as their padded entries leave room for in a stage.
-                std::int32_t rows = 0, width = 0;
-                while (rows < shape.rows && b + rows < e) {
-                    const std::int32_t wider = std::max(width, (cut.count[order[b + rows]] + 1) / 2 * 2);
-                    if (rows > 0 && (rows + 1) * wider > shape.entries) break;
-                    width = wider;
-                    ++rows;
-                }
-                if (width > 0xff) return false;
-                cut.task.insert(cut.task.end(), {0, at, rows | width << 8, 0});
-                for (std::int32_t l = 0; l < rows; ++l) cut.place[order[b + l]] = at + l;
-                const std::int32_t padded = (rows + shape.pad - 1) / shape.pad * shape.pad;
-                cut.rows.insert(cut.rows.end(), order.begin() + b, order.begin() + b + rows);
-                cut.rows.insert(cut.rows.end(), static_cast<std::size_t>(padded - rows), -1);
-                at += padded;
-                b += rows;
+            // As many rows as their padded entries leave room for in a stage.
+            std::int32_t rows = 0, width = 0;
+            while (rows < shape.rows && b + rows < e) {
+                const std::int32_t wider = std::max(width, (cut.count[order[b + rows]] + 1) / 2 * 2);
+                if (rows > 0 && (rows + 1) * wider > shape.entries) break;
+                width = wider;
+                ++rows;
             }
+            if (width > 0xff) return false;
+            cut.pieces.push_back({b, rows, width, b + rows == e});
+            b += rows;
         }
     }
-    cut.rows.resize(cut.rows.size() + 32, -1);   // a task's copies always take 32 places
     return true;
+}
+
+// The tasks into steps; a level's last step is filled up with tasks of no rows.
+void cut_steps(Cut& cut, const Sweep& sweep, std::size_t owned, const Shape& shape)
+{
+    const std::size_t tasks = cut.pieces.size() + static_cast<std::size_t>(shape.warps - 1) * sweep.depth;
+    cut.place.allocate(owned);
+    cut.task.reserve(4 * tasks);
+    cut.rows.reserve(owned + static_cast<std::size_t>(shape.pad) * tasks + 32);
+    std::int32_t at = 0;
+    auto add = [&](std::int32_t packed) {
+        for (const std::int32_t word : {0, at, packed, 0}) cut.task.push_back(word);
+    };
+    for (const Cut::Piece& q : cut.pieces) {
+        const std::int32_t padded = (q.rows + shape.pad - 1) / shape.pad * shape.pad;
+        add(q.rows | q.width << 8);
+        const auto first = sweep.h_order.begin() + q.first;
+        for (std::int32_t l = 0; l < q.rows; ++l) cut.place[first[l]] = at + l;
+        cut.rows.insert(cut.rows.end(), first, first + q.rows);
+        cut.rows.insert(cut.rows.end(), static_cast<std::size_t>(padded - q.rows), -1);
+        at += padded;
+        while (q.ends && cut.task.size() / 4 % shape.warps != 0) add(0);
+    }
+    cut.rows.resize(cut.rows.size() + 32, -1);   // a task's copies always take 32 places
 }
 
 // A direction's tables on the host.
@@ -1007,21 +1033,84 @@ struct Planned {
 constexpr int teams_of(int warps) { return warps == 1 ? kTeams1 : warps == 2 ? kTeams2 : kTeams4; }
 Shape component_shape(int warps) { return Shape{warps, 32, kTaskEntries, 4, false, teams_of(warps)}; }
 
-// ring_rows: 0 for as many as shared memory holds.
-bool plan_local(Planned& x, LocalSweep& lo, LocalSweep& up, const Sweep& lower, const Sweep& upper, std::size_t owned,
-                int warps, std::size_t element_size, int ring_rows, const std::int32_t* lower_begin,
-                const std::int32_t* lower_end, const std::int32_t* upper_begin, const std::int32_t* upper_end,
-                const std::int32_t* cols)
+// Warps per team of the cheapest shape, or 0 when the level-scheduled sweep is
+// cheaper.  A shape costs the steps that it cuts the levels into, at their
+// measured times on meshes (an ILU step of one, two and four tasks 75, 95 and
+// 145 ns, an SSOR step, which divides, 95, 130 and 172 ns), 35 ns more for a
+// step of tasks wider than six dependencies (which also hold 24 rows, not 32,
+// so there are more of them), and in SSOR the copy of the values that precedes
+// every apply, 4 ps a value beyond what the other sweep reads.  Against it stand
+// 800 ns a level for ILU (0.71 to 0.86 us measured at 250 to 1,400 rows a level)
+// and 870 ns for SSOR, once for every eight entries of a row, which that sweep
+// reads in rounds of eight.  FP32 SSOR takes three quarters of these step times,
+// and the figures for its copies and levels are in the same scale (6 ps; a level
+// 575 ns with 3 entries a row, 710 to 760 with 7).  Levels of equal width,
+// this / level-scheduled, ns a level on the two sides of the line:
+//   ILU, 3 dependencies a row: 640 rows 636 / 774, 700 rows 789 / 788; 7 of
+//   them: 384 rows 718 / 794, 512 rows 991 / 819;
+//   SSOR, 3 of them, bs 1: 640 rows 858 / 890, 700 rows 6 steps / 891; bs 64:
+//   128 rows 433 / 1,013, 512 rows 1,579 / 1,324; FP32, bs 1: 640 rows
+//   667 / 696, 700 rows 6 steps / 721.
+// FP32 and stored ILU factors cross where FP64 ones do, both sides a tenth to a
+// fifth cheaper.
+int local_sweep_warps(const Cut& lower_cut, const Cut& upper_cut, const Sweep& lower, const Sweep& upper,
+                      std::size_t owned, std::size_t bs, std::size_t element_size, int sm_count, bool ssor)
 {
+    static constexpr struct { int warps; double ilu, ssor; } kShapes[] = {{1, 75, 95}, {2, 95, 130}, {4, 145, 172}};
+    constexpr double kWide = 35;
+    if (bs > static_cast<std::size_t>(sm_count)) return 0;
+    double cost[3] = {0, 0, 0}, entries = 0;
+    for (const Cut* cut : {&lower_cut, &upper_cut}) {
+        for (std::size_t r = 0; r < owned; ++r) entries += cut->count.data[r];
+        std::int32_t tasks = 0, wide = 0;
+        for (const Cut::Piece& q : cut->pieces) {
+            ++tasks;
+            wide += q.width > 6;
+            if (!q.ends) continue;
+            for (int k = 0; k < 3; ++k)
+                cost[k] += (tasks + kShapes[k].warps - 1) / kShapes[k].warps
+                    * ((ssor ? kShapes[k].ssor : kShapes[k].ilu) + kWide * wide / tasks);
+            tasks = wide = 0;
+        }
+    }
+    const bool wide_values = element_size == 8;
+    const double copy = ssor ? (wide_values ? 0.004 : 0.006) * entries * static_cast<double>(bs) : 0;
+    const double per_row = entries / static_cast<double>(owned) + 1;
+    const double round = wide_values ? 870 : std::min(940.0, 618 + 45 * per_row);
+    double least = (ssor ? round * std::ceil(per_row / 8) : 800.0) * (lower.depth + upper.depth) - copy;
+    int best = 0;
+    for (int k = 0; k < 3; ++k)
+        if (cost[k] < least) {
+            least = cost[k];
+            best = kShapes[k].warps;
+        }
+    return best;
+}
+
+// False where the level-scheduled sweep is cheaper, or a direction does not suit
+// the schedule.  ring_rows: 0 for as many as shared memory holds.
+bool plan_local(Planned& x, LocalSweep& lo, LocalSweep& up, const Sweep& lower, const Sweep& upper, std::size_t owned,
+                std::size_t bs, std::size_t element_size, int sm_count, int ring_rows, const std::int32_t* lower_begin,
+                const std::int32_t* lower_end, const std::int32_t* upper_begin, const std::int32_t* upper_end,
+                const std::int32_t* cols, bool ssor)
+{
+    if (owned == 0) return false;
+    if (!both(owned, [&] { return count_dependencies(x.lower, owned, lower_begin, lower_end, cols, false)
+                                && cut_tasks(x.lower, lower, owned, component_shape(1)); },
+              [&] { return count_dependencies(x.upper, owned, upper_begin, upper_end, cols, true)
+                        && cut_tasks(x.upper, upper, owned, component_shape(1)); })) return false;
+    const int warps = local_sweep_warps(x.lower, x.upper, lower, upper, owned, bs, element_size, sm_count, ssor);
+    if (warps == 0) return false;
     const Shape shape = component_shape(warps);
     if (ring_rows == 0) {
         const std::size_t stage = element_size == 8 ? sizeof(Stage<double>) : sizeof(Stage<float>);
         const std::size_t stages = static_cast<std::size_t>(warps * shape.teams * kDepth) * stage;
         ring_rows = static_cast<int>((kSharedBytes - stages) / element_size) - 2;
     }
-    return both(owned, [&] { return cut_steps(x.lower, lower, owned, lower_begin, lower_end, cols, false, shape); },
-                [&] { return cut_steps(x.upper, upper, owned, upper_begin, upper_end, cols, true, shape); })
-        && both(owned, [&] { return plan_direction(x.lower_plan, lo, owned, lower, x.lower, x.upper, lower_begin, lower_end,
+    both(owned, [&] { return cut_steps(x.lower, lower, owned, shape), true; },
+         [&] { return cut_steps(x.upper, upper, owned, shape), true; });
+    return both(owned,
+                [&] { return plan_direction(x.lower_plan, lo, owned, lower, x.lower, x.upper, lower_begin, lower_end,
                                             cols, false, shape, ring_rows); },
                 [&] { return plan_direction(x.upper_plan, up, owned, upper, x.upper, x.lower, upper_begin, upper_end,
                                             cols, true, shape, ring_rows); });
@@ -1054,50 +1143,22 @@ void place_direction(Context& ctx, LocalSweep& s, const Plan& plan, const Cut& c
 
 }  // namespace
 
-// Warps per team of the cheapest shape, or 0 when the level-scheduled sweep is
-// cheaper: the steps of each shape at their measured cost against 800 ns a
-// level (0.71 to 0.86 us measured at 250 to 1,400 rows a level).  The line lies
-// at about 700 rows a level, where both take 0.8 us.
-int local_sweep_warps(int sm_count, const Sweep& lower, const Sweep& upper, std::size_t owned, std::size_t bs)
-{
-    static constexpr struct { int warps; double ns; } kShapes[] = {{1, 75}, {2, 95}, {4, 145}};
-    const char* env = std::getenv("OWTK_LOCAL_SWEEP");   // 0: never
-    if (env && std::atoi(env) == 0) return 0;
-    if (owned == 0 || bs > static_cast<std::size_t>(sm_count)) return 0;
-    std::vector<std::size_t> size;
-    for (const Sweep* s : {&lower, &upper}) {
-        const std::size_t at = size.size();
-        size.resize(at + static_cast<std::size_t>(s->depth), 0);
-        for (std::size_t r = 0; r < owned; ++r) ++size[at + static_cast<std::size_t>(s->h_level[r])];
-    }
-    double least = 800.0 * static_cast<double>(size.size());
-    int best = 0;
-    for (const auto& k : kShapes) {
-        double cost = 0;
-        for (const std::size_t rows : size)
-            cost += static_cast<double>((rows + 32 * k.warps - 1) / (32 * k.warps)) * k.ns;
-        if (cost < least) {
-            least = cost;
-            best = k.warps;
-        }
-    }
-    return best;
-}
-
 // Dependencies of row r: entries [lower_begin[r], lower_end[r]) with a column
 // below r, and [upper_begin[r], upper_end[r]) with one above it.
-void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t element_size,
-                       const std::int32_t* lower_begin, const std::int32_t* lower_end, const std::int32_t* upper_begin,
-                       const std::int32_t* upper_end, const std::int32_t* cols, bool ssor)
+void build_local_sweep(Context& ctx, Preconditioner& p, std::size_t element_size, const std::int32_t* lower_begin,
+                       const std::int32_t* lower_end, const std::int32_t* upper_begin, const std::int32_t* upper_end,
+                       const std::int32_t* cols, bool ssor)
 {
-    const Shape shape = component_shape(warps);
+    const char* env = std::getenv("OWTK_LOCAL_SWEEP");   // 0: never
+    if (env && std::atoi(env) == 0) return;
     Planned x;
-    if (!plan_local(x, p.lower_local, p.upper_local, p.lower, p.upper, p.owned, warps, element_size, 0, lower_begin,
-                    lower_end, upper_begin, upper_end, cols)) {
+    if (!plan_local(x, p.lower_local, p.upper_local, p.lower, p.upper, p.owned, p.bs, element_size, ctx.sm_count, 0,
+                    lower_begin, lower_end, upper_begin, upper_end, cols, ssor)) {
         p.lower_local = LocalSweep();
         p.upper_local = LocalSweep();
         return;
     }
+    const Shape shape = component_shape(p.lower_local.warps);
     place_direction(ctx, p.lower_local, x.lower_plan, x.lower, p.bs, element_size, element_size, ssor, shape);
     place_direction(ctx, p.upper_local, x.upper_plan, x.upper, p.bs, element_size, element_size, true, shape);
 }
@@ -1117,18 +1178,18 @@ owtk_local_schedule local_schedule(const LocalSweep& lower, const LocalSweep& up
 
 // No CUDA call.
 owtk_local_schedule plan_local_schedule(std::size_t owned, std::size_t bs, const std::int32_t* rowptr,
-                                        const std::int32_t* cols, std::size_t element_size, int sm_count, int ring_rows)
+                                        const std::int32_t* cols, std::size_t element_size, int sm_count, int ring_rows,
+                                        bool ssor)
 {
     std::vector<std::int32_t> lower_level, upper_level;
     levels_of(owned, rowptr, cols, lower_level, upper_level);
     Sweep lower, upper;
     order_by_level(lower, owned, bs, lower_level);
     order_by_level(upper, owned, bs, upper_level);
-    const int warps = local_sweep_warps(sm_count, lower, upper, owned, bs);
     LocalSweep lo, up;
     Planned x;
-    if (warps == 0 || !plan_local(x, lo, up, lower, upper, owned, warps, element_size, ring_rows, rowptr, rowptr + 1,
-                                  rowptr, rowptr + 1, cols)) return {};
+    if (!plan_local(x, lo, up, lower, upper, owned, bs, element_size, sm_count, ring_rows, rowptr, rowptr + 1, rowptr,
+                    rowptr + 1, cols, ssor)) return {};
     return local_schedule(lo, up);
 }
 
@@ -1210,12 +1271,15 @@ void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage
     std::vector<std::int32_t> after(n);   // first upper entry of each row
     for (std::size_t r = 0; r < n; ++r) after[r] = dp[r] + 1;
     Cut lower, upper;
-    if (!both(n, [&] { return cut_steps(lower, p.lower, n, rp, dp, ci, false, shape); },
-              [&] { return cut_steps(upper, p.upper, n, after.data(), rp + 1, ci, true, shape); })) return;
-    const std::size_t tasks = (lower.task.size() + upper.task.size()) / 4;
+    if (!both(n, [&] { return count_dependencies(lower, n, rp, dp, ci, false) && cut_tasks(lower, p.lower, n, shape); },
+              [&] { return count_dependencies(upper, n, after.data(), rp + 1, ci, true)
+                        && cut_tasks(upper, p.upper, n, shape); })) return;
+    const std::size_t tasks = lower.pieces.size() + upper.pieces.size();
     const double task_ns = kBlockTaskNs[storage == OWTK_F64 ? 2 : storage == OWTK_F32 ? 1 : 0][bs - 1];
     const double level_ns = storage == OWTK_F64 ? 1400.0 : 1100.0;
     if (static_cast<double>(tasks) * task_ns > level_ns * (p.lower.depth + p.upper.depth)) return;
+    both(n, [&] { return cut_steps(lower, p.lower, n, shape), true; },
+         [&] { return cut_steps(upper, p.upper, n, shape), true; });
     Plan lower_plan, upper_plan;
     if (!both(n, [&] { return plan_direction(lower_plan, p.lower_local, n, p.lower, lower, upper, rp, dp, ci, false, shape,
                                           shared_rows); },

@@ -355,14 +355,14 @@ void build_cluster_sweep(Context& ctx, ClusterSweep& s, std::size_t owned, std::
                          const std::vector<std::int32_t>& level, const std::vector<std::int32_t>& rowptr,
                          const std::vector<std::int32_t>& cols, const std::vector<std::int32_t>& diagpos,
                          bool backward, std::vector<std::uint32_t>& loc);
-int local_sweep_warps(int sm_count, const Sweep& lower, const Sweep& upper, std::size_t owned, std::size_t bs);
-void build_local_sweep(Context& ctx, Preconditioner& p, int warps, std::size_t element_size,
-                       const std::int32_t* lower_begin, const std::int32_t* lower_end, const std::int32_t* upper_begin,
-                       const std::int32_t* upper_end, const std::int32_t* cols, bool ssor);
+void build_local_sweep(Context& ctx, Preconditioner& p, std::size_t element_size, const std::int32_t* lower_begin,
+                       const std::int32_t* lower_end, const std::int32_t* upper_begin, const std::int32_t* upper_end,
+                       const std::int32_t* cols, bool ssor);
 void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage);
 owtk_local_schedule local_schedule(const LocalSweep& lower, const LocalSweep& upper);
 owtk_local_schedule plan_local_schedule(std::size_t owned, std::size_t bs, const std::int32_t* rowptr,
-                                        const std::int32_t* cols, std::size_t element_size, int sm_count, int ring_rows);
+                                        const std::int32_t* cols, std::size_t element_size, int sm_count, int ring_rows,
+                                        bool ssor);
 void rcm_order(std::size_t owned, const std::int32_t* rowptr, const std::int32_t* cols,
                std::uint64_t* out);
 void hilbert_order(std::size_t n, const double* xy, std::uint64_t* out);

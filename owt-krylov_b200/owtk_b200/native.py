@@ -134,7 +134,8 @@ def lib():
             "owtk_inverse_permutation": (c_int, [sz, vp, vp]),
             "owtk_level_sets": (c_int, [sz, vp, vp, vp, vp, u64p, u64p]),
             "owtk_pc_local_schedule": (c_int, [vp, POINTER(LocalSchedule)]),
-            "owtk_local_schedule_plan": (c_int, [sz, sz, vp, vp, sz, c_int32, POINTER(LocalSchedule)]),
+            "owtk_local_schedule_plan": (c_int, [sz, sz, vp, vp, sz, c_int32, c_int32,
+                                                 POINTER(LocalSchedule)]),
             "owtk_default_options": (None, [POINTER(SolverOptions)]),
             "owtk_workspace_create": (c_int, [vp, POINTER(vp)]),
             "owtk_workspace_destroy": (c_int, [vp]),
@@ -480,11 +481,13 @@ class Preconditioner:
         return lo, up, dl.value, du.value
 
 
-def local_schedule_plan(owned: int, bs: int, rowptr, cols, element_size: int = 8, ring_rows: int = 0) -> LocalSchedule:
-    """The one-CTA-per-component schedule of a pattern's ILU(0) and SSOR applies (warps 0: another one), on the host."""
+def local_schedule_plan(owned: int, bs: int, rowptr, cols, element_size: int = 8, ssor: bool = False,
+                        ring_rows: int = 0) -> LocalSchedule:
+    """The one-CTA-per-component schedule of a pattern's ILU(0) or SSOR applies (warps 0: another one), on the host."""
     rp, ci = _u64(rowptr), _u64(cols)
     out = LocalSchedule()
-    check(lib().owtk_local_schedule_plan(owned, bs, _ptr(rp), _ptr(ci), element_size, ring_rows, ctypes.byref(out)))
+    check(lib().owtk_local_schedule_plan(owned, bs, _ptr(rp), _ptr(ci), element_size, int(ssor), ring_rows,
+                                         ctypes.byref(out)))
     return out
 
     def close(self):

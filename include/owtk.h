@@ -225,6 +225,10 @@ typedef struct owtk_local_schedule {
     int32_t slow_tasks;     /* tasks with longer rows, or more far values, than a stage holds */
     int32_t far_steps;      /* least number of steps that a far value lies back; INT32_MAX without any */
 } owtk_local_schedule;
+/* Whether an ILU preconditioner's numeric factorisation waits for the factor
+ * values themselves (short rows, narrow levels) or for a flag per row.  The
+ * same bits either way. */
+owtk_status owtk_pc_factor_by_value(owtk_preconditioner* pc, int32_t* by_value);
 /* The schedule that an ILU, SSOR or block ILU preconditioner's applies run on. */
 owtk_status owtk_pc_local_schedule(owtk_preconditioner* pc, owtk_local_schedule* out);
 /* The schedule that ILU(0) or (ssor != 0) SSOR applies of this pattern take,

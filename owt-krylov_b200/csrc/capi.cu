@@ -241,7 +241,6 @@ void ilu_symbolic(Preconditioner& p, const Matrix& m, std::size_t fill)
     p.d_upd_start = upload(s, start);
     p.d_upd_target = upload(s, target);
     p.d_upd_upper = upload(s, upper);
-    kern::build_factor_programs(*p.ctx, p);
     const std::size_t per = p.block ? p.bs * p.bs : p.bs;   // values per factor entry
     p.d_fvalues.allocate(nnz * per * dsize(p.dtype) + 16);
     p.inv_diag.allocate(n * per * dsize(p.dtype) + 16);
@@ -249,6 +248,7 @@ void ilu_symbolic(Preconditioner& p, const Matrix& m, std::size_t fill)
     std::vector<std::int32_t> lower_level, upper_level;
     levels_of(n, p.f_rowptr.data(), p.f_cols.data(), lower_level, upper_level);
     build_sweep(*p.ctx, p.lower, n, p.bs, lower_level, false);
+    kern::build_factor_programs(*p.ctx, p);
     build_sweep(*p.ctx, p.upper, n, p.bs, upper_level, true);
     if (!p.block) {
         build_chain_sweep(*p.ctx, p.chain, n, p.lower.depth, p.upper.depth, p.f_rowptr);
@@ -1266,6 +1266,14 @@ owtk_status owtk_ilu_factors(owtk_preconditioner* pc, uint64_t* entries, uint64_
         if (inverse_diagonal)
             OWTK_CUDA(cudaMemcpyAsync(inverse_diagonal, pc->inv_diag.ptr, pc->owned * per * es, cudaMemcpyDeviceToHost, pc->ctx->stream));
         pc->ctx->sync();
+    });
+}
+
+owtk_status owtk_pc_factor_by_value(owtk_preconditioner* pc, int32_t* by_value)
+{
+    return guarded([&] {
+        require(pc != nullptr && by_value != nullptr, "null handle");
+        *by_value = pc->d_prog_start.ptr != nullptr;
     });
 }
 

@@ -971,20 +971,32 @@ template<class T> void fill_sentinel(Context& c, std::size_t n, T* x)
     c.launched();
 }
 
-// The programs of k_ilu_factor, for component-diagonal factors whose rows fit.
+// The programs of k_ilu_factor, for component-diagonal factors whose rows fit
+// and whose levels are narrow enough.  A half warp per (row, component) shortens
+// a level, but is more work than a warp that takes 32 components of its rows, so
+// wide levels of many components keep the flags.  The two cross where a level
+// has about 6,000 tasks (a task: two components of a row) with one lower entry a
+// row, 12,000 with two, 15,000 with three, 22,000 with five and 32,000 with
+// seven; the line lies at 4,500 tasks a lower entry.  20 levels, flags / values:
+// 375 rows a level, bs 16, 3 lower entries 263 / 149 us; 5,000 rows 1,131 /
+// 1,393 us; 1,250 rows, bs 64, 1 lower entry 306 / 674 us; a 2M-vertex mesh of
+// bs 3 (700 tasks a level) 132 / 47 ms.
 void build_factor_programs(Context& c, Preconditioner& p)
 {
     if (p.block) return;
     const std::size_t n = p.owned;
     std::vector<std::int32_t> start(n + 1, 0);
-    std::int64_t total = 0;
+    std::int64_t total = 0, lower_entries = 0;
     for (std::size_t r = 0; r < n; ++r) {
         const std::int32_t lower = p.f_diagpos[r] - p.f_rowptr[r], len = p.f_rowptr[r + 1] - p.f_rowptr[r];
         if (len > kFactorRow || lower > kFactorLower) return;
         total += lower * len;
+        lower_entries += lower;
         if (total >= INT32_MAX) return;
         start[r + 1] = static_cast<std::int32_t>(total);
     }
+    const double tasks = static_cast<double>(n * ((p.bs + 1) / 2));
+    if (tasks * n > 4500.0 * lower_entries * p.lower.depth) return;
     p.d_prog_start = upload(c.stream, start);
     p.d_program.allocate(static_cast<std::size_t>(total) * 4 + 16);
     k_factor_program<<<static_cast<unsigned>((n + kThreads - 1) / kThreads), kThreads, 0, c.stream>>>(

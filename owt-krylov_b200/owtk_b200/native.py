@@ -133,6 +133,7 @@ def lib():
             "owtk_hilbert_order": (c_int, [sz, vp, vp]),
             "owtk_inverse_permutation": (c_int, [sz, vp, vp]),
             "owtk_level_sets": (c_int, [sz, vp, vp, vp, vp, u64p, u64p]),
+            "owtk_pc_factor_by_value": (c_int, [vp, POINTER(c_int32)]),
             "owtk_pc_local_schedule": (c_int, [vp, POINTER(LocalSchedule)]),
             "owtk_local_schedule_plan": (c_int, [sz, sz, vp, vp, sz, c_int32, c_int32,
                                                  POINTER(LocalSchedule)]),
@@ -465,6 +466,12 @@ class Preconditioner:
         w = c_int32()
         check(lib().owtk_pc_chain_schedule(self.h, ctypes.byref(w)))
         return w.value
+
+    def factor_by_value(self) -> bool:
+        """Whether the ILU factorisation waits for values rather than flags."""
+        out = c_int32()
+        check(lib().owtk_pc_factor_by_value(self.h, ctypes.byref(out)))
+        return bool(out.value)
 
     def local_schedule(self) -> LocalSchedule:
         """The schedule with one CTA per component (warps 0: the applies take another sweep)."""

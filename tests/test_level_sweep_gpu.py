@@ -131,3 +131,32 @@ def test_cluster_schedules_equal_level_scheduled(native, ctx, problems, by_level
     assert getattr(cluster, query)()[0] > 0 and cluster.local_schedule().warps == 0
     x = np.random.default_rng(7).uniform(-1, 1, n * 3).astype(dtype)
     assert_bitwise(_apply(native, ctx, cluster, n, 3, x), _apply(native, ctx, levels, n, 3, x), env)
+
+
+# Tasks (two components of a row) a level on both sides of 4,500 for each lower
+# entry of the mean row (0.83, 2.5 and 1.67 of them here).
+@pytest.mark.parametrize("width,lower,bs,by_value", [(400, 1, 16, True), (600, 1, 16, False), (1100, 3, 20, True),
+                                                     (1500, 3, 20, False), (150, 1, 64, False), (300, 2, 33, True)])
+def test_factors_by_value_or_flag(native, ctx, restatement, width, lower, bs, by_value):
+    depth = 6
+    n = width * depth
+    r = np.arange(n)
+    e = []
+    for d in range(lower):
+        some = r[(r >= width) & (r % width + d < width)]
+        e.append(np.stack([some, some - width + d], 1))
+    e = np.concatenate(e)
+    rows, cols = np.concatenate([r, e[:, 0], e[:, 1]]), np.concatenate([r, e[:, 1], e[:, 0]])
+    o = np.lexsort((cols, rows))
+    rows, cols = rows[o], cols[o]
+    rp = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(rows, minlength=n), out=rp[1:])
+    v = -np.random.default_rng(width).uniform(0.05, 1.0, size=(cols.size, bs))
+    v[rows == cols] = 2.5 * lower
+    m = native.Matrix(ctx, "bsr", n, 0, bs, rp, cols, v.reshape(-1))
+    p = native.Preconditioner(m, native.PC_ILU, 0)
+    assert p.factor_by_value() == by_value
+    _, _, values, inverse = p.ilu_factors()
+    want = restatement.ilu(n, bs, rp, cols, v.reshape(-1), 0).factors()
+    assert_bitwise(values, want[2], "factors")
+    assert_bitwise(inverse, want[3], "inverse diagonal")

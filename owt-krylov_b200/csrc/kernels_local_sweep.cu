@@ -783,14 +783,6 @@ template<class T> struct Table {
     T& operator[](std::size_t i) { return data[i]; }
 };
 
-template<class T> DeviceBuffer upload_table(cudaStream_t stream, const Table<T>& host)
-{
-    DeviceBuffer b(host.size * sizeof(T) + 16);
-    if (host.size > 0)
-        OWTK_CUDA(cudaMemcpyAsync(b.ptr, host.data.get(), host.size * sizeof(T), cudaMemcpyHostToDevice, stream));
-    return b;
-}
-
 // A direction's rows in step order, padded: each task starts at a multiple of
 // four places.
 struct Cut {
@@ -1116,28 +1108,50 @@ bool plan_local(Planned& x, LocalSweep& lo, LocalSweep& up, const Sweep& lower, 
                                             cols, true, shape, ring_rows); });
 }
 
-// The plan on the device.  vector_size, value_size: bytes of a vector element
-// and of a stored value.
+// The plan on the device, in one allocation (with one for each of the twenty
+// parts of both directions this took 4.2 of the 7 ms that the tables of 90,000
+// rows take on the host).
+// vector_size, value_size: bytes of a vector element and of a stored value.
 void place_direction(Context& ctx, LocalSweep& s, const Plan& plan, const Cut& cut, std::size_t bs,
                      std::size_t vector_size, std::size_t value_size, bool with_fin, const Shape& shape)
 {
-    s.task = upload(ctx.stream, cut.task);
-    s.slots = upload_table(ctx.stream, plan.slots);
-    if (!plan.far.empty()) s.far = upload(ctx.stream, plan.far);
-    if (!plan.code.empty()) s.code = upload(ctx.stream, plan.code);
-    s.src = upload_table(ctx.stream, plan.src);
-    s.rows = upload(ctx.stream, cut.rows);
-    s.to = upload_table(ctx.stream, plan.to);
     // Values of an entry, and of a row's diagonal.
     const std::size_t per = !shape.block ? bs : value_size == 2 ? (bs * bs + 1) / 2 * 2 : bs * bs;
-    s.coef.allocate(per * s.entries * value_size + 16);
-    OWTK_CUDA(cudaMemsetAsync(s.coef.ptr, 0, per * s.entries * value_size, ctx.stream));   // padding: zero
-    if (with_fin) {
-        s.fin.allocate(per * s.places * value_size + 16);
-        OWTK_CUDA(cudaMemsetAsync(s.fin.ptr, 0, per * s.places * value_size, ctx.stream));
+    std::size_t total = 0;
+    auto room = [&](std::size_t bytes) {   // a part's offset; a copy may read 16 bytes past its end
+        const std::size_t at = total;
+        total += (bytes + 16 + 255) / 256 * 256;
+        return at;
+    };
+    struct Copy {
+        DevicePart& part;
+        const void* from;
+        std::size_t bytes, at;
+    };
+    std::vector<Copy> copies;
+    auto copied = [&](DevicePart& part, const void* from, std::size_t bytes) {
+        if (bytes > 0) copies.push_back({part, from, bytes, room(bytes)});
+    };
+    copied(s.task, cut.task.data(), cut.task.size() * 4);
+    copied(s.slots, plan.slots.data.get(), plan.slots.size * 2);
+    copied(s.far, plan.far.data(), plan.far.size() * 4);
+    copied(s.code, plan.code.data(), plan.code.size() * 4);
+    copied(s.src, plan.src.data.get(), plan.src.size * 4);
+    copied(s.rows, cut.rows.data(), cut.rows.size() * 4);
+    copied(s.to, plan.to.data.get(), plan.to.size * 4);
+    const std::size_t zeroed = total, coef = room(per * s.entries * value_size),   // padding: zero
+                      fin = with_fin ? room(per * s.places * value_size) : 0,
+                      in = room(bs * s.places * vector_size);
+    s.store.allocate(total);
+    char* base = s.store.as<char>();
+    for (const Copy& c : copies) {
+        c.part.ptr = base + c.at;
+        OWTK_CUDA(cudaMemcpyAsync(c.part.ptr, c.from, c.bytes, cudaMemcpyHostToDevice, ctx.stream));
     }
-    s.in.allocate(bs * s.places * vector_size + 16);
-    OWTK_CUDA(cudaMemsetAsync(s.in.ptr, 0, bs * s.places * vector_size, ctx.stream));
+    s.coef.ptr = base + coef;
+    if (with_fin) s.fin.ptr = base + fin;
+    s.in.ptr = base + in;
+    OWTK_CUDA(cudaMemsetAsync(base + zeroed, 0, total - zeroed, ctx.stream));
     s.ready = true;
 }
 
@@ -1232,8 +1246,8 @@ void launch_block(Context& c, Preconditioner& p, T* out)
 }
 
 template<class F, bool DIAG>
-void pack_blocks(Context& c, const LocalSweep& s, std::size_t bs, const DeviceBuffer& src, const F* from,
-                 const DeviceBuffer& to)
+void pack_blocks(Context& c, const LocalSweep& s, std::size_t bs, const DevicePart& src, const F* from,
+                 const DevicePart& to)
 {
     const std::size_t tasks = static_cast<std::size_t>(s.steps) * s.warps;
     k_local_block_pack<F, DIAG><<<static_cast<unsigned>((tasks * 32 + kThreads - 1) / kThreads), kThreads, 0, c.stream>>>(

@@ -66,6 +66,12 @@ struct DeviceBuffer {
     template<class T> T* as() const { return static_cast<T*>(ptr); }
 };
 
+// A part of a DeviceBuffer.
+struct DevicePart {
+    void* ptr = nullptr;
+    template<class T> T* as() const { return static_cast<T*>(ptr); }
+};
+
 // Upload a host vector into a fresh device buffer (synchronous on the stream).
 template<class T>
 DeviceBuffer upload(cudaStream_t s, const std::vector<T>& host)
@@ -255,16 +261,17 @@ struct LocalSweep {
     int slow_tasks = 0;
     std::size_t entries = 0;   // padded
     std::size_t places = 0;    // padded rows
-    DeviceBuffer task;         // int4 per step and warp: first entry, first place, rows and width (and flags), ring slot
-    DeviceBuffer slots;        // uint16 per entry, the two of a pair side by side: ring slot or staged far value
-    DeviceBuffer far;          // 32 int32 per task, if any task has one: dependencies beyond the ring's reach
-    DeviceBuffer code;         // int32 per entry, if any task needs it: ring slot or far dependency
-    DeviceBuffer src;          // int32 per entry: factor or matrix entry (-1: padding)
-    DeviceBuffer rows;         // int32 per place: row (-1: padding)
-    DeviceBuffer to;           // int32 per place: its place in the other direction's order (forward only)
-    DeviceBuffer coef;         // per component and entry
-    DeviceBuffer fin;          // per component and place: what scales or divides the result
-    DeviceBuffer in;           // per component and place: right-hand side, or the forward result
+    DeviceBuffer store;        // what the parts below lie in
+    DevicePart task;           // int4 per step and warp: first entry, first place, rows and width (and flags), ring slot
+    DevicePart slots;          // uint16 per entry, the two of a pair side by side: ring slot or staged far value
+    DevicePart far;            // 32 int32 per task, if any task has one: dependencies beyond the ring's reach
+    DevicePart code;           // int32 per entry, if any task needs it: ring slot or far dependency
+    DevicePart src;            // int32 per entry: factor or matrix entry (-1: padding)
+    DevicePart rows;           // int32 per place: row (-1: padding)
+    DevicePart to;             // int32 per place: its place in the other direction's order (forward only)
+    DevicePart coef;           // per component and entry
+    DevicePart fin;            // per component and place: what scales or divides the result
+    DevicePart in;             // per component and place: right-hand side, or the forward result
 };
 struct Preconditioner {
     Context* ctx = nullptr;

@@ -1045,10 +1045,18 @@ Shape component_shape(int warps) { return Shape{warps, 32, kTaskEntries, 4, fals
 //   667 / 696, 700 rows 6 steps / 721.
 // FP32 and stored ILU factors cross where FP64 ones do, both sides a tenth to a
 // fifth cheaper.
+constexpr struct { int warps; double ilu, ssor; } kShapes[] = {{1, 75, 95}, {2, 95, 130}, {4, 145, 172}};
+
+// What the level-scheduled sweep takes for a level, ns, by entries per row.
+double level_ns(double per_row, std::size_t element_size, bool ssor)
+{
+    if (!ssor) return 800;
+    return std::ceil(per_row / 8) * (element_size == 8 ? 870 : std::min(940.0, 618 + 45 * per_row));
+}
+
 int local_sweep_warps(const Cut& lower_cut, const Cut& upper_cut, const Sweep& lower, const Sweep& upper,
                       std::size_t owned, std::size_t bs, std::size_t element_size, int sm_count, bool ssor)
 {
-    static constexpr struct { int warps; double ilu, ssor; } kShapes[] = {{1, 75, 95}, {2, 95, 130}, {4, 145, 172}};
     constexpr double kWide = 35;
     if (bs > static_cast<std::size_t>(sm_count)) return 0;
     double cost[3] = {0, 0, 0}, entries = 0;
@@ -1065,11 +1073,9 @@ int local_sweep_warps(const Cut& lower_cut, const Cut& upper_cut, const Sweep& l
             tasks = wide = 0;
         }
     }
-    const bool wide_values = element_size == 8;
-    const double copy = ssor ? (wide_values ? 0.004 : 0.006) * entries * static_cast<double>(bs) : 0;
+    const double copy = ssor ? (element_size == 8 ? 0.004 : 0.006) * entries * static_cast<double>(bs) : 0;
     const double per_row = entries / static_cast<double>(owned) + 1;
-    const double round = wide_values ? 870 : std::min(940.0, 618 + 45 * per_row);
-    double least = (ssor ? round * std::ceil(per_row / 8) : 800.0) * (lower.depth + upper.depth) - copy;
+    double least = level_ns(per_row, element_size, ssor) * (lower.depth + upper.depth) - copy;
     int best = 0;
     for (int k = 0; k < 3; ++k)
         if (cost[k] < least) {
@@ -1087,6 +1093,11 @@ bool plan_local(Planned& x, LocalSweep& lo, LocalSweep& up, const Sweep& lower, 
                 const std::int32_t* cols, bool ssor)
 {
     if (owned == 0) return false;
+    // Wide levels are told without cutting them: no cut is cheaper than full
+    // steps of four tasks, no row longer than all its entries.
+    const double rows = static_cast<double>(owned), full = 2 * rows / 128 * (ssor ? kShapes[2].ssor : kShapes[2].ilu);
+    if (full >= level_ns((lower_end[owned - 1] - lower_begin[0]) / rows, element_size, ssor) * (lower.depth + upper.depth))
+        return false;
     if (!both(owned, [&] { return count_dependencies(x.lower, owned, lower_begin, lower_end, cols, false)
                                 && cut_tasks(x.lower, lower, owned, component_shape(1)); },
               [&] { return count_dependencies(x.upper, owned, upper_begin, upper_end, cols, true)

@@ -781,8 +781,9 @@ __global__ void __launch_bounds__(kThreads) k_norm(std::size_t n, const T* __res
 // BiCGSTAB's two vector updates with the norm that follows each, in one pass
 // and one launch: the updated vector is reduced from registers instead of
 // being read back, and at small sizes, where a launch and the host's wait for
-// a scalar are most of the time, an iteration has two launches fewer.  The
-// norms only meet thresholds; the dots stay in their own kernel, because a
+// a scalar are most of the time, an iteration has two launches fewer.  Here
+// the norms only meet thresholds (other solvers scale vectors by k_norm's); the
+// dots stay in their own kernel, because a
 // differently compiled copy of its loop contracts other products into fused
 // multiply-adds and the iteration amplifies the last bit of rho (the final
 // residual of a 12,288-unknown Jacobi solve then moves in its second to

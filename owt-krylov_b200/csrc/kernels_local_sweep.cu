@@ -1276,9 +1276,12 @@ template<class T, class F> std::size_t block_stage_bytes(std::size_t bs)
 }  // namespace
 
 // The dense-block ILU's schedule where it pays: its tasks at their cost (BF16,
-// FP32 and FP64 factors, by block size; measured at 82 rows a level, a step
-// being one task) against what a level costs through L2 (1.15 us for FP32
-// vectors, 1.5 us for FP64).
+// FP32 and FP64 factors, by block size; fitted at 82 rows a level, a step being
+// one task) against what a level costs through L2 (1.1 us for FP32 vectors,
+// 1.4 us for FP64).  At 1 to 320 rows a level of 1, 3 and 7 dependencies a row
+// nothing taken is slower than the level-scheduled sweep (ns a level, this /
+// that, BF16 bs 3: 32 rows 185 / 1,084, 192 rows 875 / 1,164; FP64 bs 3: 32 rows
+// 396 / 1,381; FP64 bs 4: 32 rows 641 / 1,335).
 constexpr double kBlockTaskNs[3][4] = {{105, 110, 160, 210}, {105, 110, 140, 310}, {105, 140, 390, 700}};
 void build_local_block_sweep(Context& ctx, Preconditioner& p, owtk_dtype storage)
 {

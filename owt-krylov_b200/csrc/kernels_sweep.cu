@@ -3,7 +3,8 @@
 //
 // This is the schedule for wide levels.  While the levels are narrow, ILU and
 // SSOR applies run on one CTA per component instead (kernels_local_sweep.cu),
-// and rows of up to 16 entries are factorised by k_ilu_factor below, which
+// and rows of up to 16 entries in levels that are not too wide for it
+// (build_factor_programs) are factorised by k_ilu_factor below, which
 // synchronises on the factor's values.
 //
 // Schedule (built once at symbolic setup, reused by every numeric update and
@@ -783,8 +784,8 @@ __global__ void __launch_bounds__(kThreads) k_sweep(SweepArgs<T, F> a)
 // the subtractions of one pivot step run side by side and a level costs one L2
 // hand-off plus a division and a shuffle per lower entry; indices and matrix
 // values are loaded, and all operands polled at once, before the first step.
-// For rows of up to 16 entries and 8 lower ones; others keep per-row flags
-// (row_body), behind which the values are read one by one.  50,000 rows, bs 4,
+// For rows of up to 16 entries and 8 lower ones; others, and very wide levels,
+// keep per-row flags (row_body), behind which the values are read one by one.  50,000 rows, bs 4,
 // 871 levels: 11.1 ms with the flags, 3.3 ms with one lane per (row, component)
 // and the row in shared memory, 1.7 ms so.
 constexpr int kFactorRow = 16;        // lanes of a (row, component)
